@@ -27,7 +27,7 @@
 #include <string>
 #include <vector>
 
-#include "internal.cuh"
+#include "batch.cuh"
 #include "jterms.cuh"
 #include "reduce.cuh"
 #include "sector.cuh"
@@ -102,12 +102,6 @@ __device__ __forceinline__ T hx_jterms(const BatchTables<T> &tb, const Sec<T> &s
     return (T)h;
 }
 
-template <int CL>
-__device__ __forceinline__ int cta_rank() {
-    if constexpr (CL == 1) return 0;
-    else return (int)cg::this_cluster().block_rank();
-}
-
 // Sum of NS compensated partials over the job's CTAs, returned in every
 // thread of every CTA.  Cluster partials are double-buffered: a buffer is
 // written again only two sums later, after every CTA has passed the barrier
@@ -151,50 +145,8 @@ __device__ __forceinline__ void job_sum(CSum (&a)[NS], BatchSmem<T> &sm, double 
     __syncthreads();
 }
 
-// Next job of the queue for this CTA (CL == 1) or cluster (rank 0 takes it,
-// the others read it from rank 0's shared memory).  The closing barrier
-// keeps rank 0 from exiting or overwriting the slot before every CTA read it.
-template <int CL, typename T>
-__device__ __forceinline__ int next_job(unsigned *queue, BatchSmem<T> &sm) {
-    if constexpr (CL == 1) {
-        if (threadIdx.x == 0) sm.job = (int)atomicAdd(queue, 1u);
-        __syncthreads();
-        const int j = sm.job;
-        __syncthreads();
-        return j;
-    } else {
-        cg::cluster_group cl = cg::this_cluster();
-        if (cl.block_rank() == 0 && threadIdx.x == 0) sm.job = (int)atomicAdd(queue, 1u);
-        cl.sync();
-        if (threadIdx.x == 0) sm.jobl = *cl.map_shared_rank(&sm.job, 0);
-        cl.sync();
-        return sm.jobl;
-    }
-}
-
 // ---------------------------------------------------------------- chains --
-struct ChainJob {
-    int tnup, tndw;        // target sector
-    int snup;              // source sector's nup (down-spin sign)
-    int ispin, iorb, particle;
-    int kmax;
-    int slot;              // output slot
-    int64_t psi_off;       // FP64 state vector in the eigenspace pool
-    int64_t work_off;      // elements of T: three vectors of the job
-};
-
-// Chain output slot: alpha[kLzMax+2], beta[kLzMax+2], then nsteps and norm2
-// in separate arrays.
-constexpr int kChainStride = kLzMax + 2;
-
 // One chain, run by CL CTAs (a cluster) or by one CTA.
-// Extents of the buffers a batched launch writes or gathers from, checked
-// against every job in a checked build (the checks are uniform over the CTAs
-// of a cluster, so a skipped job is skipped by all of them).
-struct BatchCaps {
-    int64_t work, vec, aux, states, slots, lock;
-};
-
 template <typename T, int CL>
 __device__ void chain_job(const BatchTables<T> &tb, BatchSmem<T> &sm, const ChainJob &J,
                           const double *states64, T *work, double *alpha, double *beta,
@@ -325,18 +277,6 @@ __global__ void __launch_bounds__(kBatchThreads, 1)
 }
 
 // ------------------------------------------------------------ eigensolve --
-struct EigsJob {
-    int nup, ndw;
-    int neigen, kmax;
-    int slot;          // output slot: evals, steps
-    int64_t basis_off; // elements of T: (kmax + 1) vectors of ld elements
-    int64_t vec_off;   // FP64 eigenvectors: neigen x dim
-    int64_t aux_off;   // FP64 scratch: Y and coefficients (2 x neigen x kmax)
-    int64_t lock_off;  // locked FP64 vectors (dim apart) in the lock pool
-    int nlock;         // how many (0: plain run)
-    double top;        // probe: eigenvalues above this are not wanted (early stop)
-};
-
 constexpr int kEigsChunk = 4;  // basis vectors per reorthogonalisation dot pass
 constexpr int kMaxWaves = 64;  // launches of one batched eigensolve (memory budget)
 constexpr double kDgks = 0.717;  // second Gram-Schmidt pass below this norm ratio
@@ -871,41 +811,6 @@ void gf_add_chain(dmfted_ctx *c, int nlanc, const double *alanc, const double *b
         }
 }
 
-// Persistent launch: as many CTAs (CL == 1) or clusters as can be resident,
-// at most one per job.
-template <typename... KArgs, typename... Args>
-static void launch_persistent(dmfted_ctx *c, void (*kern)(KArgs...), int CL, int njobs,
-                              size_t smem, Args &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kBatchThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CL;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = CL > 1 ? 1 : 0;
-    if (CL > 8) {
-        // 16 CTAs per cluster is beyond the portable size: opt in per kernel
-        DM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    }
-    int units = std::max(1, num_sms(c) / CL);
-    if (CL > 1) {
-        cfg.gridDim = dim3(units * CL);
-        int ncl = 0;
-        if (cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) == cudaSuccess && ncl > 0)
-            units = ncl;
-        else
-            (void)cudaGetLastError();
-    }
-    units = std::min(units, njobs);
-    cfg.gridDim = dim3(units * CL);
-    DM_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
-    c->launches++;
-}
-
 // CTAs per eigensolve job: from the largest sector (at least
 // batch_cluster_min states per CTA, to amortise the cluster barriers; 16, the
 // non-portable cluster size, from 32 per CTA: on the Ns=10 workload, whose
@@ -922,9 +827,11 @@ static int eigs_cluster(const dmfted_ctx *c, int64_t dmax) {
 }
 
 // CTAs per chain: two once the largest chain holds 16 x batch_cluster_min
-// states (the long chains set the phase's time: 200 chains of the Ns=10
-// workload took 35.0 ms with pairs against 38.9 ms one per CTA), more only
-// while the chains leave SMs idle; or DMFTED_BATCH_CLUSTER_GF.
+// states (the long chains set the phase's time: with the vectors in L2, 200
+// chains of the Ns=10 workload took 35.0 ms with pairs against 38.9 ms one per
+// CTA), more only while the chains leave SMs idle; or DMFTED_BATCH_CLUSTER_GF.
+// On-chip chains take at least the CTAs their largest needs (four at 52,920
+// states: 8.8 ms; eight 11.3 ms).
 static int chain_cluster(dmfted_ctx *c, int njobs, int64_t dmax) {
     const int64_t per = c->batch_cluster_min;
     if (const char *e = getenv("DMFTED_BATCH_CLUSTER_GF")) {
@@ -1023,7 +930,8 @@ static void run_batch_eigs(dmfted_ctx *c, int j0, int nbig, int j1, int wave, do
                                      (int)eigs_smem()));
         attr[c->device & 63] = true;
     }
-    launch_persistent(c, k_batch_eigs<T, CL>, CL, nbig + div_up(j1 - j0 - nbig, CL), eigs_smem(),
+    launch_persistent(c, k_batch_eigs<T, CL>, CL, nbig + div_up(j1 - j0 - nbig, CL), kBatchThreads,
+                      eigs_smem(),
                       batch_tables<T>(c), reinterpret_cast<const EigsJob *>(c->bjobs.p) + j0, nbig,
                       j1 - j0, reinterpret_cast<unsigned *>(c->bint.p) + 2 * wave,
                       reinterpret_cast<T *>(c->bwork.p), c->bvec.p, c->baux.p, c->bscal.p,
@@ -1176,7 +1084,7 @@ void batch_eigs(dmfted_ctx *c, const std::vector<int> &list, const std::vector<i
 template <typename T, int CL>
 static void run_batch_chains(dmfted_ctx *c, int nbig, int nj, double *alpha, double *beta,
                              int *nsteps, double *norm2, int64_t nslots) {
-    launch_persistent(c, k_batch_chains<T, CL>, CL, nbig + div_up(nj - nbig, CL), 0,
+    launch_persistent(c, k_batch_chains<T, CL>, CL, nbig + div_up(nj - nbig, CL), kBatchThreads, 0,
                       batch_tables<T>(c), reinterpret_cast<const ChainJob *>(c->bjobs.p), nbig, nj,
                       reinterpret_cast<unsigned *>(c->bint.p), (const double *)c->states64.p,
                       reinterpret_cast<T *>(c->bwork.p), alpha, beta, nsteps, norm2,
@@ -1265,21 +1173,32 @@ void batch_chains_gf(dmfted_ctx *c, const std::vector<ChainRec> &recs, int preci
     const size_t cf_off = round_up(std::max<size_t>(jobs.size(), 1) * sizeof(ChainJob), 256);
     c->bjobs.alloc(cf_off + nrec * sizeof(ChainCF));
     if (!jobs.empty()) {
-        c->bwork.alloc(work * es);
         std::stable_sort(jobs.begin(), jobs.end(), [&](const ChainJob &a, const ChainJob &b) {
             const double ca = (double)c->binom[a.tnup] * c->binom[a.tndw] * a.kmax;
             const double cb = (double)c->binom[b.tnup] * c->binom[b.tndw] * b.kmax;
             return ca > cb;
         });
-        int64_t dmax = 0;
+        // on chip: FP64 chains without Jhflag terms whose vectors fit a
+        // cluster's shared memory and registers; the rest through L2
+        std::vector<ChainJob> onchip, rest;
         for (const ChainJob &J : jobs)
-            dmax = std::max<int64_t>(dmax, c->binom[J.tnup] * c->binom[J.tndw]);
-        tuned_cluster(c, "chains", "DMFTED_BATCH_CLUSTER_GF",
-                      chain_cluster(c, (int)jobs.size(), dmax), (int64_t)jobs.size(), dmax,
-                      fp64 ? DMFTED_FP64 : DMFTED_MIXED, [&](int cl) {
-                          if (fp64) run_batch_chains_cl<double>(c, cl, jobs, alpha, beta, nsteps, norm2, nrec);
-                          else run_batch_chains_cl<float>(c, cl, jobs, alpha, beta, nsteps, norm2, nrec);
-                      });
+            (fp64 && !c->jterms && oc_need(c, J.tnup, J.tndw) > 0 ? onchip : rest).push_back(J);
+        if (!rest.empty()) c->bwork.alloc(work * es);
+        const int prec = fp64 ? DMFTED_FP64 : DMFTED_MIXED;
+        for (const std::vector<ChainJob> *part : {&onchip, &rest}) {
+            if (part->empty()) continue;
+            int64_t dmax = 0;
+            for (const ChainJob &J : *part)
+                dmax = std::max<int64_t>(dmax, c->binom[J.tnup] * c->binom[J.tndw]);
+            const bool oc = part == &onchip;
+            tuned_cluster(c, oc ? "chains" : "chains-L2", "DMFTED_BATCH_CLUSTER_GF",
+                          chain_cluster(c, (int)part->size(), dmax), (int64_t)part->size(), dmax,
+                          prec, [&](int cl) {
+                              if (oc) run_chains_onchip(c, cl, *part, alpha, beta, nsteps, norm2, nrec);
+                              else if (fp64) run_batch_chains_cl<double>(c, cl, *part, alpha, beta, nsteps, norm2, nrec);
+                              else run_batch_chains_cl<float>(c, cl, *part, alpha, beta, nsteps, norm2, nrec);
+                          });
+        }
     }
     // chains too large for one CTA: the grid-wide recurrence, two at a time
     // (the second on the second lane) so that each chain's kernels fill the

@@ -29,6 +29,7 @@ struct BatchTables {
     int64_t poff[kMaxNs + 1];   // padded class offsets
     int64_t binom[kMaxNs + 1];  // class sizes
     int64_t nrank;              // entries of the rank table (2^Ns)
+    uint8_t hmax[2][kMaxNs + 1];  // most hops of a word, per spin and class
     int norb, P, W;
     double jx, jp;              // Jhflag spin-exchange / pair hopping (0: none)
 };
@@ -42,6 +43,8 @@ inline BatchTables<T> batch_tables(const dmfted_ctx *c) {
         const SpinTables &t = (s == 1 && !c->spin_shared) ? c->spin[1] : c->spin[0];
         b.sp[s].cnt = t.cnt.p;
         b.sp[s].ell = t.ell.p;
+        for (int n = 0; n <= c->ns; n++)
+            b.hmax[s][n] = (uint8_t)((int)t.cls_max.size() > n ? t.cls_max[n] : std::max(c->W, 1));
         if constexpr (sizeof(T) == 8) {
             b.sp[s].diag = (const T *)t.diag.p;
             b.sp[s].par = (const T *)t.par.p;
