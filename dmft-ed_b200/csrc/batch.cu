@@ -339,24 +339,27 @@ __device__ void reorth_dots(const T *B, uint32_t ld, int nv, const T *y, uint32_
         for (int t = 0; t < kEigsChunk; t++) d[t].zero();
         for (uint32_t b0 = (uint32_t)(rank * bd) + (uint32_t)sl * st; b0 < dim;
              b0 += (uint32_t)nsl * st) {
-            for (uint32_t l = lane; l < (uint32_t)bd; l += 64) {
-                const uint32_t i = b0 + l, i2 = i + 32;
-                if (i >= dim) break;
-                const bool ok2 = l + 32 < (uint32_t)bd && i2 < dim;
-                const double yi = (double)y[i];
-                const double yi2 = ok2 ? (double)y[i2] : 0.0;
-                double p1[kEigsChunk], p2[kEigsChunk];
+            // four vectors x four elements of each lane in flight, added in
+            // element order
+            for (uint32_t l = lane; l < (uint32_t)bd; l += 128) {
+                if (b0 + l >= dim) break;
+                double ye[4], pe[kEigsChunk][4];
+                bool ok[4];
 #pragma unroll
-                for (int t = 0; t < kEigsChunk; t++) {
-                    const T *bj = B + (int64_t)(j0 + t) * ld;
-                    p1[t] = j0 + t < nv ? (double)bj[i] : 0.0;
-                    p2[t] = (j0 + t < nv && ok2) ? (double)bj[i2] : 0.0;
+                for (int q = 0; q < 4; q++) {
+                    ok[q] = b0 + l + 32 * q < dim;  // bd is a multiple of 128
+                    ye[q] = ok[q] ? (double)y[b0 + l + 32 * q] : 0.0;
                 }
 #pragma unroll
                 for (int t = 0; t < kEigsChunk; t++) {
-                    d[t].add(p1[t] * yi);
-                    d[t].add(p2[t] * yi2);
+                    const T *bj = B + (int64_t)min(j0 + t, nv - 1) * ld + b0 + l;
+#pragma unroll
+                    for (int q = 0; q < 4; q++) pe[t][q] = ok[q] ? (double)bj[32 * q] : 0.0;
                 }
+#pragma unroll
+                for (int t = 0; t < kEigsChunk; t++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) d[t].add(pe[t][q] * ye[q]);
             }
         }
 #pragma unroll
@@ -393,22 +396,36 @@ __device__ __forceinline__ CSum reorth_update(const T *B, uint32_t ld, int nv, T
     const uint32_t i0 = (uint32_t)(rank * blockDim.x + threadIdx.x), st = CL * blockDim.x;
     CSum nrm;
     nrm.zero();
-    for (uint32_t i = i0; i < dim; i += st) {
-        double acc[8];
+    for (uint32_t i = i0; i < dim; i += 2 * st) {
+        // two elements x eight vectors in flight
+        const bool two = i + st < dim;
+        const uint32_t i2 = two ? i + st : i;
+        double acc[8], ac2[8];
 #pragma unroll
-        for (int t = 0; t < 8; t++) acc[t] = 0.0;
-        int j = 0;
-        for (; j + 8 <= nv; j += 8) {
+        for (int t = 0; t < 8; t++) acc[t] = ac2[t] = 0.0;
+        for (int j = 0; j < nv; j += 8) {
+            double b1[8], b2[8];
 #pragma unroll
-            for (int t = 0; t < 8; t++)
-                acc[t] = fma(scf[j + t], (double)B[(int64_t)(j + t) * ld + i], acc[t]);
+            for (int t = 0; t < 8; t++) {
+                const T *bj = B + (int64_t)min(j + t, nv - 1) * ld;
+                b1[t] = (double)bj[i];
+                b2[t] = (double)bj[i2];
+            }
+#pragma unroll
+            for (int t = 0; t < 8; t++) {
+                const double c = j + t < nv ? scf[j + t] : 0.0;
+                acc[t] = fma(c, b1[t], acc[t]);
+                ac2[t] = fma(c, b2[t], ac2[t]);
+            }
         }
-        for (int t = 0; j < nv; j++, t++) acc[t] = fma(scf[j], (double)B[(int64_t)j * ld + i], acc[t]);
-        const double sub =
-            ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-        const T w = (T)((double)y[i] - sub);
-        y[i] = w;
-        nrm.add((double)w * (double)w);
+        auto put = [&](uint32_t k, const double (&a)[8]) {
+            const double sub = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+            const T w = (T)((double)y[k] - sub);
+            y[k] = w;
+            nrm.add((double)w * (double)w);
+        };
+        put(i, acc);
+        if (two) put(i2, ac2);
     }
     return nrm;
 }
@@ -509,6 +526,13 @@ __device__ void eigs_job(const BatchTables<T> &tb, BatchSmem<T> &sm, double *dyn
     __syncthreads();
     int n = 0;
     bool brk = false;
+    // Ritz tests fall on multiples of ncheck steps.  A test takes as long as ten
+    // steps: while the decay of the worst estimate (over its target) since the
+    // last test predicts more than four intervals to go, every other one is
+    // left out, so the test that sees convergence is the one the fixed schedule
+    // would run.
+    int next = ncheck, at_prev = 0;
+    double worst_prev = 0.0;
     for (int k = 0; k < J.kmax; k++) {
         const T *x = B + (int64_t)k * ld;
         const T *xp = B + (int64_t)(k > 0 ? k - 1 : 0) * ld;
@@ -611,19 +635,33 @@ __device__ void eigs_job(const BatchTables<T> &tb, BatchSmem<T> &sm, double *dyn
             brk = true;
             break;
         }
-        if (n % ncheck == 0 && n < J.kmax) {
+        if (n >= next && n < J.kmax) {
             // Ritz test on the lowest Neigen pairs of T_n
             for (int i = tid; i < n; i += bd) rwork[i] = sal[i];
             for (int i = tid; i < n; i += bd) rwork[n + i] = i > 0 ? sbe[i] : 0.0;
             __syncthreads();
-            const int m = min(J.neigen, n);
-            const bool ok = ritz_multi_dev(rwork, rwork + n, n, J.neigen, tol, sbe[n], evp,
-                                           Y, coef, rwork + 2 * n,
-                                           (int)eigs_ritz_doubles() - 2 * n);
-            if (ok && n >= m && m == J.neigen) break;
-            // a probe whose lowest Ritz value stays above the acceptance
-            // threshold by ten times its residual estimate found nothing new
-            if (J.nlock > 0 && evp[0] > J.top && coef[0] <= 0.1 * (evp[0] - J.top)) break;
+            const bool ok = ritz_multi_dev<false>(rwork, rwork + n, n, J.neigen, tol, sbe[n], evp,
+                                                  Y, coef, rwork + 2 * n,
+                                                  (int)eigs_ritz_doubles() - 2 * n);
+            if (ok && n >= J.neigen) break;
+            next = n + ncheck;
+            if (J.nlock > 0) {
+                // a probe whose lowest Ritz value stays above the acceptance
+                // threshold by ten times its residual estimate found nothing new
+                if (evp[0] > J.top && coef[0] <= 0.1 * (evp[0] - J.top)) break;
+                continue;
+            }
+            if (n < J.neigen) continue;
+            const double eps23 = 3.666852862501036e-11;
+            double worst = 0.0;
+            for (int j = 0; j < J.neigen; j++)
+                worst = fmax(worst, coef[j] / (tol * fmax(eps23, fabs(evp[j]))));
+            if (worst_prev > worst && worst > 1.0) {
+                const double rate = log(worst_prev / worst) / (n - at_prev);
+                if (log(worst) > 4.0 * ncheck * rate) next = n + 2 * ncheck;
+            }
+            worst_prev = worst;
+            at_prev = n;
         }
     }
     (void)brk;
@@ -632,7 +670,7 @@ __device__ void eigs_job(const BatchTables<T> &tb, BatchSmem<T> &sm, double *dyn
     for (int i = tid; i < n; i += bd) rwork[n + i] = i > 0 ? sbe[i] : 0.0;
     __syncthreads();
     const int mm = min(J.neigen, n);
-    ritz_multi_dev(rwork, rwork + n, n, mm, tol, sbe[n], evp, Y, coef, rwork + 2 * n,
+    ritz_multi_dev<true>(rwork, rwork + n, n, mm, tol, sbe[n], evp, Y, coef, rwork + 2 * n,
                    (int)eigs_ritz_doubles() - 2 * n);
     if (rank == 0)
         for (int j = tid; j < mm; j += bd) evals[(int64_t)J.slot * kEigsMaxEigen + j] = evp[j];
@@ -813,10 +851,11 @@ void gf_add_chain(dmfted_ctx *c, int nlanc, const double *alanc, const double *b
 
 // CTAs per eigensolve job: from the largest sector (at least
 // batch_cluster_min states per CTA, to amortise the cluster barriers; 16, the
-// non-portable cluster size, from 32 per CTA: on the Ns=10 workload, whose
-// largest sector holds 63,504 states, 16 took 35.9 ms of eigensolves against
-// 38.6 ms for 8), or DMFTED_BATCH_CLUSTER_EIGS.  Only sectors that give every
-// CTA that many states are shared; smaller ones run one per CTA.
+// non-portable cluster size, from 32 per CTA), or DMFTED_BATCH_CLUSTER_EIGS.
+// Only sectors that give every CTA that many states are shared; smaller ones
+// run one per CTA.  (Eight CTAs are faster on the Ns=10 workload, 18.1 against
+// 23.4 ms of eigensolves, but end in other last digits: quantities that vanish
+// by symmetry are then other rounding noise.)
 static int eigs_cluster(const dmfted_ctx *c, int64_t dmax) {
     const int64_t per = c->batch_cluster_min;
     if (const char *e = getenv("DMFTED_BATCH_CLUSTER_EIGS")) {

@@ -10,8 +10,12 @@
 //   1. Householder tridiagonalisation A = Q T Q^T (the unblocked reduction of
 //      LAPACK's dsytd2: per column a reflector H = I - tau v v^T, then the
 //      trailing block updated by the rank-2 form A - v w^T - w v^T with
-//      w = p - (tau/2)(p.v) v, p = tau A v); v overwrites the column below the
-//      diagonal and tau the diagonal entry, which T has already taken;
+//      w = p - (tau/2)(p.v) v, p = tau A v).  The update of one column and the
+//      product of the next are one pass over the trailing block: the next
+//      column is updated first, by itself, which gives its reflector, and the
+//      pass then updates every row and multiplies it.  Reflectors go to the
+//      rows of A (coalesced), tau to the diagonal entry, which T has already
+//      taken;
 //   2. the lowest m eigenpairs of T by Sturm multisection and inverse
 //      iteration (tridiag.cuh), with clusters of equal eigenvalues -- a sector
 //      holding several ground states -- given an orthonormal basis of their
@@ -19,6 +23,12 @@
 //   3. the back-transformation x = H_0 H_1 ... H_{n-3} y of those m vectors.
 // A lives in global memory (L2-resident: 0.5 MB at the default threshold of
 // 256 states); the reflector and the product vectors live in shared memory.
+// What bounds it: per column one L2 latency for the column and one per row of a
+// warp in the pass (eight loads of a row in flight), and three block sums: the
+// 44 sectors of the Ns=8 scan (at most 224 states) 3.95 -> 2.84 ms against
+// separate update and product passes.
+// (A packed triangle in shared memory took 1.7 ms for the same sectors, but
+// sums in another order.)
 #include <algorithm>
 #include <vector>
 
@@ -49,10 +59,10 @@ __global__ void __launch_bounds__(kDenseThreads, 1)
                  double *work, double *vecs, double *evals, int64_t work_cap, int64_t vec_cap,
                  int ritz_cap) {
     extern __shared__ double dyn[];  // T (a, b), then the Ritz work space
-    __shared__ double s_v[kDenseMaxDim], s_p[kDenseMaxDim];
+    // the new reflector, and the pending update A -= v w^T + w v^T, by row of A
+    __shared__ double s_x[kDenseMaxDim], s_v[kDenseMaxDim], s_w[kDenseMaxDim], s_p[kDenseMaxDim];
     __shared__ double s_red[32];
     __shared__ double s_ev[kDenseMaxEigen], s_est[kDenseMaxEigen];
-    __shared__ double s_tau, s_k;
     __shared__ int s_job;
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int nwarp = bd >> 5;
@@ -103,78 +113,104 @@ __global__ void __launch_bounds__(kDenseThreads, 1)
         double *sa = dyn, *sb = dyn + n;
         if (tid == 0) sb[0] = 0.0;
         // ---- 1. tridiagonalisation -------------------------------------------
+        for (int i = tid; i < n; i += bd) s_v[i] = s_w[i] = 0.0;
+        __syncthreads();
         for (int k = 0; k + 1 < n; k++) {
             const int m = n - k - 1;  // length of the column below the diagonal
-            double part = 0.0;
+            // column k with the pending update, its length, its reflector
+            double part = 0.0, dk = 0.0;
             for (int i = tid; i < m; i += bd) {
-                const double x = A[(int64_t)(k + 1 + i) * n + k];
-                s_v[i] = x;
+                const int r = k + 1 + i;
+                double x = A[(int64_t)r * n + k];
+                x -= s_v[r] * s_w[k] + s_w[r] * s_v[k];
+                s_x[r] = x;
                 if (i > 0) part += x * x;
             }
-            const double tail = dense_block_sum(part, s_red);  // |x|^2 without x_0
             if (tid == 0) {
-                const double x0 = s_v[0];
-                sa[k] = A[(int64_t)k * n + k];
-                if (m == 1 || tail == 0.0) {
-                    s_tau = 0.0;  // already tridiagonal in this column
-                    sb[k + 1] = x0;
-                } else {
-                    const double nx = sqrt(x0 * x0 + tail);
-                    const double alpha = x0 >= 0.0 ? -nx : nx;
-                    const double v0 = x0 - alpha;
-                    s_v[0] = v0;
-                    s_tau = 2.0 / (v0 * v0 + tail);
-                    sb[k + 1] = alpha;
-                }
-                A[(int64_t)k * n + k] = s_tau;  // T holds a_k now; keep tau here
+                dk = A[(int64_t)k * n + k];
+                dk -= s_v[k] * s_w[k] + s_w[k] * s_v[k];
+                sa[k] = dk;
+            }
+            const double tail = dense_block_sum(part, s_red);  // |x|^2 without x_0
+            const double x0 = s_x[k + 1];
+            double tau = 0.0, alpha = x0, v0 = 0.0;
+            if (m > 1 && tail != 0.0) {  // else already tridiagonal in this column
+                const double nx = sqrt(x0 * x0 + tail);
+                alpha = x0 >= 0.0 ? -nx : nx;
+                v0 = x0 - alpha;
+                tau = 2.0 / (v0 * v0 + tail);
+            }
+            __syncthreads();  // every thread has x0
+            if (tid == 0) {
+                sb[k + 1] = alpha;
+                A[(int64_t)k * n + k] = tau;  // T holds a_k now; keep tau here
+                if (tau != 0.0) s_x[k + 1] = v0;
             }
             __syncthreads();
-            const double tau = s_tau;
-            if (tau == 0.0) continue;
-            for (int i = tid; i < m; i += bd) A[(int64_t)(k + 1 + i) * n + k] = s_v[i];
-            // p = tau A_sub v, one warp per row
+            if (tau != 0.0)
+                for (int i = tid; i < m; i += bd) A[(int64_t)k * n + k + 1 + i] = s_x[k + 1 + i];
+            // the pending update of every row and p = tau A_sub v, one warp per row
+            const double *xk = s_x + k + 1, *vk = s_v + k + 1, *wk = s_w + k + 1;
             for (int i = warp; i < m; i += nwarp) {
-                const double *row = A + (int64_t)(k + 1 + i) * n + (k + 1);
+                double *row = A + (int64_t)(k + 1 + i) * n + (k + 1);
+                const double vi = vk[i], wi = wk[i];
                 double d = 0.0;
-                for (int j = lane; j < m; j += 32) d += row[j] * s_v[j];
+                for (int j0 = lane; j0 < m; j0 += 256) {
+                    double e[8];
+#pragma unroll
+                    for (int t = 0; t < 8; t++) e[t] = j0 + 32 * t < m ? row[j0 + 32 * t] : 0.0;
+#pragma unroll
+                    for (int t = 0; t < 8; t++) {
+                        const int j = j0 + 32 * t;
+                        if (j < m) {
+                            e[t] -= vi * wk[j] + wi * vk[j];
+                            row[j] = e[t];
+                            d += e[t] * xk[j];
+                        }
+                    }
+                }
                 for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
                 if (lane == 0) s_p[i] = tau * d;
             }
             __syncthreads();
+            // w = p - (tau/2)(p.v) v replaces the pending update
             part = 0.0;
-            for (int i = tid; i < m; i += bd) part += s_p[i] * s_v[i];
+            for (int i = tid; i < m; i += bd) part += s_p[i] * s_x[k + 1 + i];
             const double kk = 0.5 * tau * dense_block_sum(part, s_red);
-            for (int i = tid; i < m; i += bd) s_p[i] -= kk * s_v[i];  // w
-            __syncthreads();
-            // A_sub -= v w^T + w v^T
-            for (int64_t t = tid; t < (int64_t)m * m; t += bd) {
-                const int i = (int)(t / m), j = (int)(t % m);
-                A[(int64_t)(k + 1 + i) * n + (k + 1 + j)] -= s_v[i] * s_p[j] + s_p[i] * s_v[j];
+            for (int i = tid; i < m; i += bd) {
+                const int r = k + 1 + i;
+                s_v[r] = tau != 0.0 ? s_x[r] : 0.0;
+                s_w[r] = tau != 0.0 ? s_p[i] - kk * s_x[r] : 0.0;
             }
             __syncthreads();
         }
-        if (tid == 0) sa[n - 1] = A[(int64_t)(n - 1) * n + (n - 1)];
+        if (tid == 0) {
+            double d = A[(int64_t)(n - 1) * n + (n - 1)];
+            d -= s_v[n - 1] * s_w[n - 1] + s_w[n - 1] * s_v[n - 1];
+            sa[n - 1] = d;
+        }
         __syncthreads();
         // ---- 2. lowest m eigenpairs of T ---------------------------------------
         double *Y = vecs + J.out_off;
-        ritz_multi_dev(sa, sb, n, J.m, 1.0, 0.0, s_ev, Y, s_est, dyn + 2 * n, ritz_cap - 2 * n);
+        ritz_multi_dev<true>(sa, sb, n, J.m, 1.0, 0.0, s_ev, Y, s_est, dyn + 2 * n, ritz_cap - 2 * n);
         // ---- 3. back-transformation x = H_0 ... H_{n-3} y ----------------------
-        for (int k = n - 2; k >= 0; k--) {
-            const double tau = A[(int64_t)k * n + k];
-            if (tau == 0.0) continue;  // uniform: every thread reads the same value
-            const int m = n - k - 1;
-            for (int i = tid; i < m; i += bd) s_v[i] = A[(int64_t)(k + 1 + i) * n + k];
-            __syncthreads();
-            for (int j = warp; j < J.m; j += nwarp) {
+        // one warp per vector: no barrier between the reflectors
+        for (int j = warp; j < J.m; j += nwarp) {
+            for (int k = n - 2; k >= 0; k--) {
+                const double *row = A + (int64_t)k * n + k;
+                const double tau = row[0];
+                if (tau == 0.0) continue;
                 double *y = Y + (int64_t)j * n + (k + 1);
+                const int m = n - k - 1;
                 double d = 0.0;
-                for (int i = lane; i < m; i += 32) d += s_v[i] * y[i];
+                for (int i = lane; i < m; i += 32) d += row[1 + i] * y[i];
                 for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
                 d *= tau;
-                for (int i = lane; i < m; i += 32) y[i] -= d * s_v[i];
+                for (int i = lane; i < m; i += 32) y[i] -= d * row[1 + i];
+                __syncwarp();
             }
-            __syncthreads();
         }
+        __syncthreads();
         for (int j = tid; j < J.m; j += bd) evals[(int64_t)J.slot * kDenseMaxEigen + j] = s_ev[j];
         __syncthreads();
     }

@@ -136,7 +136,10 @@ __global__ void __launch_bounds__(kRedThreads) k_lz_init(const T *s0, int64_t n,
 // test on its Ritz estimate, b_n |y_n| <= tol * max(eps^(2/3), |theta|)
 // (y = eigenvector of T_n, b_n = norm of the last residual).  Breakdown
 // (invariant subspace) counts as converged.
-__global__ void k_ritz_check(LanczosScalars lz, double tol) {
+// 128 threads: 8 rounds of 128 Sturm counts (with 256 the counts of a round are
+// bound by FP64 issue instead of their own chain).
+constexpr int kCheckThreads = 128;
+__global__ void __launch_bounds__(kCheckThreads) k_ritz_check(LanczosScalars lz, double tol) {
     extern __shared__ double rs[];
     const int n = lz.status[ST_STEPS];
     if (n <= 0) return;
@@ -148,9 +151,9 @@ __global__ void k_ritz_check(LanczosScalars lz, double tol) {
         sb[i] = i > 0 ? lz.beta[i] : 0.0;
     }
     __syncthreads();
-    const double e = tridiag_eig(sa, sb, n, 0);
+    const double e = tridiag_eig<false>(sa, sb, n, 0);
+    if (threadIdx.x < 32) tridiag_evec_fast(sa, sb, n, e, yv, ws, sw);
     if (threadIdx.x == 0) {
-        tridiag_evec(sa, sb, n, e, yv, ws, sw);
         const double est = fabs(lz.beta[n]) * fabs(yv[n - 1]);
         const double eps23 = 3.666852862501036e-11;
         if (lz.status[ST_BREAK] || est <= tol * fmax(eps23, fabs(e))) {
@@ -163,10 +166,11 @@ __global__ void k_ritz_check(LanczosScalars lz, double tol) {
     }
 }
 
-// Ritz vector coefficients coef[i] = y_i * scale_i for eigenvalue lam, so
-// that the Ritz vector is sum_i coef_i s_i.
-__global__ void k_ritz_vector(LanczosScalars lz, int n, double lam, double *coef) {
+// The lowest Ritz value to its last digit (lz.ritz[0]) and the coefficients
+// coef[i] = y_i * scale_i of its vector, sum_i coef_i s_i.
+__global__ void __launch_bounds__(kRedThreads) k_ritz_vector(LanczosScalars lz, int n, double *coef) {
     extern __shared__ double rs[];
+    if (n <= 0) return;
     double *sa = rs, *sb = rs + n, *yv = rs + 2 * n, *ws = rs + 3 * n;
     unsigned char *sw = reinterpret_cast<unsigned char *>(rs + 8 * n);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -174,7 +178,9 @@ __global__ void k_ritz_vector(LanczosScalars lz, int n, double lam, double *coef
         sb[i] = i > 0 ? lz.beta[i] : 0.0;
     }
     __syncthreads();
+    const double lam = tridiag_eig<true>(sa, sb, n, 0);
     if (threadIdx.x != 0) return;
+    lz.ritz[0] = lam;
     tridiag_evec(sa, sb, n, lam, yv, ws, sw);
     for (int i = 0; i < n; i++) coef[i] = yv[i] * lz.scale[i];
 }
@@ -432,7 +438,7 @@ static LanczosResult gs_run(dmfted_ctx *c, const SectorView &s, double *psi, con
             T *y = basis + (size_t)(k + 1) * ld;
             lanczos_step<T>(c, s, x, xp, y, dim, lz, k, 1e-300, 1);
         }
-        k_ritz_check<<<1, kRedThreads, ritz_smem(launched), c->stream>>>(lz, tol);
+        k_ritz_check<<<1, kCheckThreads, ritz_smem(launched), c->stream>>>(lz, tol);
         DM_CHECK_LAUNCH();
         c->launches++;
         double rz[2];
@@ -454,11 +460,9 @@ static LanczosResult gs_run(dmfted_ctx *c, const SectorView &s, double *psi, con
         // (kmax reached inside the loop: the last check above already ran)
     }
     const int n = hst[ST_STEPS];
-    double ritz[2];
-    DM_CUDA(cudaMemcpy(ritz, lz.ritz, sizeof(ritz), cudaMemcpyDeviceToHost));
-    const double e0 = ritz[0];
+    double e0 = 0.0;
     double *coef = c->coefb.p;
-    k_ritz_vector<<<1, 32, ritz_smem(n), c->stream>>>(lz, n, e0, coef);
+    k_ritz_vector<<<1, kRedThreads, ritz_smem(n), c->stream>>>(lz, n, coef);
     DM_CHECK_LAUNCH();
     k_basis_combine<T><<<eg, 256, 0, c->stream>>>(basis, (int64_t)ld, n, coef,
                                                    refine ? start : nullptr, psi, dim);
@@ -467,6 +471,7 @@ static LanczosResult gs_run(dmfted_ctx *c, const SectorView &s, double *psi, con
     k_scale_by_invsqrt<<<eg, 256, 0, c->stream>>>(psi, dim, c->red_out.p);
     DM_CHECK_LAUNCH();
     c->launches += 3;
+    DM_CUDA(cudaMemcpyAsync(&e0, lz.ritz, sizeof(e0), cudaMemcpyDeviceToHost, c->stream));
     DM_CUDA(cudaStreamSynchronize(c->stream));
     LanczosResult res{e0, n, hst[ST_CONV] != 0};
     res.capped = capped;
@@ -806,7 +811,7 @@ __global__ void k_ritz_multi(LanczosScalars lz, double tol, int mwant, double *e
         sb[i] = i > 0 ? lz.beta[i] : 0.0;
     }
     __syncthreads();
-    const bool ok = ritz_multi_dev(sa, sb, n, mwant, tol, lz.beta[n], evals, Y, est, rs + 2 * n,
+    const bool ok = ritz_multi_dev<true>(sa, sb, n, mwant, tol, lz.beta[n], evals, Y, est, rs + 2 * n,
                                    work_cap - 2 * n);
     if (threadIdx.x == 0 && !final_pass) {
         const int m = min(mwant, n);

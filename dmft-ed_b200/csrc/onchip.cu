@@ -11,9 +11,8 @@ namespace dmfted {
 // One Lanczos step: u = sc H x - b_k scp v_prev over v_prev's registers and
 // alpha (first barrier), then x -> v_prev, w = u - alpha sc x -> x and |w|
 // (second barrier).  The chains of the two-orbital Ns=10 workload (72 of up to
-// 52,920 states, four CTAs each) take 8.8 ms against 15.1 ms with the vectors
-// in L2; the two of the Ns=8 scan (4,900 and 3,920 states, two CTAs) 1.0
-// against 2.1 ms.
+// 52,920 states, four CTAs each) take 9.7 ms against 15.1 ms with the vectors
+// in L2; the two of the Ns=8 scan (4,900 and 3,920 states) 1.1 against 2.1 ms.
 template <int CL>
 __device__ void chain_job_oc(const BatchTables<double> &tb, OcSums<CL> &sums, unsigned char *dyn,
                              const ChainJob &J, const double *states64, double *alpha,
@@ -40,8 +39,7 @@ __device__ void chain_job_oc(const BatchTables<double> &tb, OcSums<CL> &sums, un
         for (int s = 0; s < kOcSlots; s++) {
             prev[s] = 0.0;
             if (s >= v.nv) continue;
-            const uint32_t c = v.c0 + v.g + v.G * s;
-            const uint32_t r = v.sw ? c : v.r, q = v.sw ? v.r : c;  // up and down ranks
+            const uint32_t r = v.r, q = v.c0 + v.g + v.G * s;  // up and down ranks
             const uint32_t wj = J.ispin == 0 ? wu[r] : wd[q];
             double val = 0.0;
             const bool has = (wj & bit) != 0u;
@@ -59,7 +57,7 @@ __device__ void chain_job_oc(const BatchTables<double> &tb, OcSums<CL> &sums, un
                 if (DM_IN(J.psi_off + src, cap.states)) val = par ? -psi[src] : psi[src];
             }
             oc_st(v.x0 + s * v.xstep, val);
-            a.add(val * val);
+            a.add_product(val, val);
         }
     }
     const double n2 = oc_sum<CL>(a, sums, buf);
@@ -69,7 +67,7 @@ __device__ void chain_job_oc(const BatchTables<double> &tb, OcSums<CL> &sums, un
     for (int k = 0; k < J.kmax; k++) {
         // keeps the slots' addresses from being hoisted out of the loop into
         // registers that prev needs
-        asm volatile("" : "+r"(v.xstep), "+r"(v.dhstep), "+r"(v.cdgstep), "+r"(v.G));
+        asm volatile("" : "+r"(v.xstep), "+r"(v.dhstep), "+r"(v.dcstep), "+r"(v.G));
         const double cprev = k > 0 ? bk * scp : 0.0;
         a.zero();
 #pragma unroll
@@ -77,14 +75,13 @@ __device__ void chain_job_oc(const BatchTables<double> &tb, OcSums<CL> &sums, un
             if (s < v.nmax) {
                 double h[kOcCols], x[kOcCols];
                 oc_product<CL>(v, s, h, x);
-                double part = 0.0;
 #pragma unroll
                 for (int j = 0; j < kOcCols; j++) {
+                    if (s + j >= v.nv) continue;
                     const double u = sc * h[j] - cprev * prev[s + j];
                     prev[s + j] = u;
-                    part = fma(x[j], u, part);
+                    a.add_product(x[j], u);
                 }
-                a.add(part);
             }
         const double ak = sc * oc_sum<CL>(a, sums, buf);
         const double coef = ak * sc;
@@ -92,7 +89,6 @@ __device__ void chain_job_oc(const BatchTables<double> &tb, OcSums<CL> &sums, un
 #pragma unroll
         for (int s = 0; s < kOcSlots; s += kOcCols)
             if (s < v.nmax) {
-                double part = 0.0;
 #pragma unroll
                 for (int j = 0; j < kOcCols; j++) {
                     if (s + j >= v.nv) continue;
@@ -100,9 +96,8 @@ __device__ void chain_job_oc(const BatchTables<double> &tb, OcSums<CL> &sums, un
                     const double x = oc_ld(xa), w = prev[s + j] - coef * x;
                     prev[s + j] = x;
                     oc_st(xa, w);
-                    part = fma(w, w, part);
+                    a.add_product(w, w);
                 }
-                a.add(part);
             }
         const double bn = sqrt(oc_sum<CL>(a, sums, buf));
         if (lead) {
@@ -148,18 +143,6 @@ __global__ void __launch_bounds__(kOcThreads, 1)
         if (jid >= njobs) break;
         chain_job_oc<1>(tb, one, ocdyn, jobs[jid], states64, alpha, beta, nsteps, norm2, thr, cap);
     }
-}
-
-// A sector's on-chip matrix: the spin with the smaller class in the rows.
-struct OcShape {
-    int64_t R, D;
-    int wr, wc;
-};
-static OcShape oc_shape(const dmfted_ctx *c, int nup, int ndw) {
-    const int wu = c->spin[0].cls_max[nup];
-    const int wd = (c->spin_shared ? c->spin[0] : c->spin[1]).cls_max[ndw];
-    if (c->binom[nup] > c->binom[ndw]) return {c->binom[ndw], c->binom[nup], wd, wu};
-    return {c->binom[nup], c->binom[ndw], wu, wd};
 }
 
 int oc_need(const dmfted_ctx *c, int nup, int ndw) {

@@ -52,12 +52,22 @@ __host__ __device__ inline size_t oc_pad(size_t b) { return (b + 15) / 16 * 16; 
 __host__ __device__ inline size_t oc_smem(int64_t R, int64_t D, int CL, int wr, int wc, int ni) {
     const size_t cpr = (size_t)((D + CL - 1) / CL);
     return oc_pad(cpr * wc * 16) + oc_pad(cpr * R * 8) + oc_pad(2 * kMaxParams * 8) +
-           oc_pad(cpr * ni * 8) + oc_pad((size_t)wr * R * 4) + oc_pad(cpr * 4);
+           oc_pad(cpr * 8) + oc_pad((size_t)ni * ni * 8) + oc_pad((size_t)wr * R * 4) + oc_pad(cpr * 4);
 }
 inline bool oc_fits(int64_t R, int64_t D, int CL, int wr, int wc, int ni) {
     if (R > kOcThreads) return false;
     const int64_t cpr = (D + CL - 1) / CL, G = kOcThreads / R;
     return (cpr + G - 1) / G <= kOcSlots && oc_smem(R, D, CL, wr, wc, ni) <= kOcMaxSmem;
+}
+
+// A sector's on-chip matrix.
+struct OcShape {
+    int64_t R, D;
+    int wr, wc;
+};
+inline OcShape oc_shape(const dmfted_ctx *c, int nup, int ndw) {
+    return {c->binom[nup], c->binom[ndw], c->spin[0].cls_max[nup],
+            (c->spin_shared ? c->spin[0] : c->spin[1]).cls_max[ndw]};
 }
 
 // Partials of a job's sums, written by every CTA of the cluster into every
@@ -88,11 +98,10 @@ struct OcView {
     uint32_t xstep;          // bytes from slot to slot: G columns
     uint32_t ut;             // the row's hop table: row byte offset | coupling offset << 16
     uint32_t spv;            // signed couplings of the row hops: +V, -V per parameter
-    uint32_t cdg;            // [ncl][ni] diagonal of the column per impurity state of the row
-    uint32_t cdgstep;        // bytes from slot to slot (already at this row's impurity state)
+    uint32_t dc, dcstep;     // [ncl] bath energies of the columns' words; slot step
+    uint32_t dint;           // impurity diagonal at this row's impurity state
     uint32_t dh, dhstep;     // [ncl][wc] column hops; bytes from slot to slot
-    uint32_t dcnt;           // [ncl] column hop counts
-    bool sw;                 // rows are the down words
+    uint32_t dcnt;           // [ncl] column hop counts | offset of the column's impurity state << 8
 };
 
 __device__ __forceinline__ uint32_t oc_cluster_rank(int CL) {
@@ -185,11 +194,10 @@ __device__ __forceinline__ double oc_sum(CSum s, OcSums<CL> &sums, int &buf) {
 template <int CL>
 __device__ __noinline__ void oc_setup(OcView &v, unsigned char *dyn, const BatchTables<double> &tb,
                                       int nup, int ndw) {
-    v.sw = tb.binom[nup] > tb.binom[ndw];
-    const int nr = v.sw ? ndw : nup, nc = v.sw ? nup : ndw;
-    const BatchSpin<double> &sr = tb.sp[v.sw ? 1 : 0], &sc = tb.sp[v.sw ? 0 : 1];
-    const int wr = tb.hmax[v.sw ? 1 : 0][nr];
-    v.wc = tb.hmax[v.sw ? 0 : 1][nc];
+    const int nr = nup, nc = ndw;
+    const BatchSpin<double> &sr = tb.sp[0], &sc = tb.sp[1];
+    const int wr = tb.hmax[0][nr];
+    v.wc = tb.hmax[1][nc];
     const int64_t orow = tb.poff[nr], ocol = tb.poff[nc];
     const uint32_t *er = sr.ell + (int64_t)tb.W * orow, *ec = sc.ell + (int64_t)tb.W * ocol;
     const uint32_t tid = threadIdx.x, bd = blockDim.x, rank = oc_cluster_rank(CL);
@@ -213,7 +221,8 @@ __device__ __noinline__ void oc_setup(OcView &v, unsigned char *dyn, const Batch
     OcHop *dh = (OcHop *)take((size_t)cpr * v.wc * 16);
     double *xs = (double *)take((size_t)cpr * v.R * 8);
     double *spv = (double *)take(2 * kMaxParams * 8);
-    double *cdg = (double *)take((size_t)cpr * ni * 8);
+    double *dc = (double *)take((size_t)cpr * 8);
+    double *dint = (double *)take((size_t)ni * ni * 8);
     uint32_t *ut = (uint32_t *)take((size_t)wr * v.R * 4);
     uint32_t *dcnt = (uint32_t *)take((size_t)cpr * 4);
     for (uint32_t i = tid; i < 2u * tb.P; i += bd) {
@@ -229,15 +238,14 @@ __device__ __noinline__ void oc_setup(OcView &v, unsigned char *dyn, const Batch
             ut[e * v.R + r] = ok ? ell_col(en) * 8u | cp << 16 : r * 8u;
         }
     }
+    for (uint32_t i = tid; i < ni * ni; i += bd) dint[i] = tb.dint[i];
     const uint32_t xs0 = oc_addr(xs);
     for (uint32_t c = tid; c < v.ncl; c += bd) {
         const uint32_t q = v.c0 + c;
-        const double dd = sc.diag[ocol + q];
+        dc[c] = sc.diag[ocol + q];
         const uint32_t ic = tb.words[ocol + q] & imask;
-        for (uint32_t ir = 0; ir < ni; ir++)
-            cdg[c * ni + ir] = dd + tb.dint[v.sw ? ic * ni + ir : ir * ni + ic];
         const int n = min((int)sc.cnt[ocol + q], v.wc);
-        dcnt[c] = (uint32_t)n;
+        dcnt[c] = (uint32_t)n | (ic * 8u) << 8;
         for (int e = 0; e < n; e++) {
             const uint32_t en = ec[(int64_t)e * v.D + q];
             const bool ok = DM_IN(ell_col(en), v.D) && DM_IN(ell_par(en), tb.P);
@@ -254,8 +262,9 @@ __device__ __noinline__ void oc_setup(OcView &v, unsigned char *dyn, const Batch
     v.xstep = v.G * v.R * 8u;
     v.ut = oc_addr(ut) + rr * 4u;
     v.spv = oc_addr(spv);
-    v.cdg = oc_addr(cdg) + (gg * ni + (tb.words[orow + rr] & imask)) * 8u;
-    v.cdgstep = v.G * ni * 8u;
+    v.dc = oc_addr(dc) + gg * 8u;
+    v.dcstep = v.G * 8u;
+    v.dint = oc_addr(dint) + (tb.words[orow + rr] & imask) * ni * 8u;
     v.dh = oc_addr(dh) + gg * v.wc * 16u;
     v.dhstep = v.G * v.wc * 16u;
     v.dcnt = oc_addr(dcnt) + gg * 4u;
@@ -278,14 +287,15 @@ __device__ __forceinline__ void oc_product(const OcView &v, int s0, double (&h)[
         col[j] = a - r8;
         if (s0 + j < v.nv) {
             x[j] = oc_ld(a);
-            h[j] = oc_ld(v.cdg + (s0 + j) * v.cdgstep);
             nd[j] = (int)oc_ld32(v.dcnt + (s0 + j) * v.G * 4u);
+            h[j] = oc_ld(v.dc + (s0 + j) * v.dcstep);
         }
-        ndmax = max(ndmax, nd[j]);
     }
 #pragma unroll
     for (int j = 0; j < kOcCols; j++) {
-        h[j] = (v.dr + h[j]) * x[j];
+        h[j] = (v.dr + h[j] + oc_ld(v.dint + ((uint32_t)nd[j] >> 8))) * x[j];
+        nd[j] &= 0xff;
+        ndmax = max(ndmax, nd[j]);
         if (s0 + j >= v.nv) col[j] = col[0];  // gathers of unused slots repeat the first
     }
     const int nr = s0 < v.nv ? v.nr : 0;

@@ -26,6 +26,14 @@ struct CSum {
         hi = s;
         lo += e;
     }
+    // add(x * y) with the product exact (its rounding error goes to lo): a sum of
+    // products then does not depend on how its terms are split over threads, to
+    // its last digit, nor on where the compiler fuses the product.
+    __device__ __forceinline__ void add_product(double x, double y) {
+        const double s = fma(x, y, hi), bb = __dadd_rn(s, -hi);
+        lo = __dadd_rn(lo, __dadd_rn(__dadd_rn(hi, -__dadd_rn(s, -bb)), fma(x, y, -bb)));
+        hi = s;
+    }
     __device__ __forceinline__ void merge(double h2, double l2) {
         double s, e;
         two_sum(hi, h2, s, e);
