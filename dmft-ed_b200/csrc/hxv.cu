@@ -652,9 +652,9 @@ __global__ void __launch_bounds__(256, kRvBlocks) k_hxv_rv(const HxvArgs<T> a) {
 constexpr uint32_t kLeanZero = 255u;
 
 // MODE 0: plain product; 1: fused Lanczos step (u and its alpha).  MB: CTAs
-// of 256 threads per SM the register budget is set for.
-template <typename T, int KU, int KD, int MODE, int MB = kRvBlocks>
-__global__ void __launch_bounds__(256, MB) k_hxv_lean(const HxvArgs<T> a,
+// of NT threads per SM the register budget is set for.
+template <typename T, int KU, int KD, int MODE, int MB = kRvBlocks, int NT = 256>
+__global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
                                                     const uint32_t *__restrict__ eux) {
     constexpr bool LZ = MODE >= 1;
     constexpr int NC = 16 / sizeof(T);
@@ -898,9 +898,205 @@ __global__ void __launch_bounds__(256, MB) k_hxv_lean(const HxvArgs<T> a,
 }
 
 // ---------------------------------------------------------------------------
+// k_hxv_lean1: k_hxv_lean for an odd number of rows (or vectors not aligned to
+// two elements), where a column does not start on a two-element boundary: one
+// row per thread and pass, the same tables and the same order of every sum (and
+// so the digits of k_hxv with one-row vectors, which it replaces there).  The
+// neighbour loads of all columns are in flight before the gathers, as in
+// k_hxv_lean; padding is skipped, not multiplied by zero, so that an infinite
+// element stays in the rows it couples to.  What bounds it: the load/store pipe.
+// Ns=13 (5,6), 1287 x 1716 FP64: 22.3 us against 38.7 us (1.58 against 0.91 TB/s
+// of the two vectors).
+template <typename T, int KU, int KD, int MODE>
+__global__ void __launch_bounds__(256, 4) k_hxv_lean1(const HxvArgs<T> a,
+                                                       const uint32_t *__restrict__ eux) {
+    constexpr bool LZ = MODE >= 1;
+    constexpr int NC = 16 / sizeof(T);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ T spv[256];
+    __shared__ __align__(16) T cdg[NC][1 << kMaxNorb];
+    __shared__ __align__(16) uint32_t noff[NC][8];
+    __shared__ __align__(16) T nval[NC][8];
+    __shared__ T ndd[NC];
+    __shared__ int ncnt[NC];
+
+    if (LZ) {
+        if (a.status[0]) return;  // chain finished: every later step is a no-op
+    }
+    const int tid = threadIdx.x, bd = blockDim.x;
+    const uint32_t dimup = (uint32_t)a.dimup, dimdw = (uint32_t)a.dimdw;
+    const uint32_t ncols = dimdw * (uint32_t)a.nstack;
+    const uint32_t total = ncols * dimup;
+    (void)total;  // bounds of the checked build
+    for (int i = tid; i < 256; i += bd) {
+        T v = T(0);
+        if (i < 2 * a.P && i != (int)kLeanZero) {
+            v = a.pu[i >> 1];
+            if (i & 1) v = -v;
+        }
+        spv[i] = v;
+    }
+    const int ni = 1 << a.norb;
+    const unsigned imask = (unsigned)ni - 1u;
+    double sc = 1.0, cprev = 0.0;
+    if (LZ) {
+        sc = a.scale[a.k];
+        cprev = a.k > 0 ? a.beta[a.k] * a.scale[a.k - 1] : 0.0;
+    }
+    const T sch = (T)sc, scl = (T)(sc - (double)sch);
+    const T cph = (T)cprev, cpl = (T)(cprev - (double)cph);
+    const T *x = a.x + (int64_t)blockIdx.y * a.vstride;
+    T *y = a.y + (int64_t)blockIdx.y * a.vstride;
+    const T *xprev = LZ ? a.xprev + (int64_t)blockIdx.y * a.vstride : nullptr;
+    T *xs = reinterpret_cast<T *>(smem_raw);  // [dimup][NC]
+    CSum dot;
+    dot.zero();
+
+    for (uint32_t c0 = blockIdx.x * NC; c0 < ncols; c0 += gridDim.x * NC) {
+        const int nc = (int)min((uint32_t)NC, ncols - c0);
+        __syncthreads();
+        for (uint32_t r = tid; r < dimup; r += bd) {
+            T v[NC];
+#pragma unroll
+            for (int j = 0; j < NC; j++) {
+                const uint32_t idx = (c0 + j) * dimup + r;
+                v[j] = j < nc && DM_IN(idx, total) ? x[idx] : T(0);
+            }
+            if (DM_IN(r * NC + NC - 1, dimup * NC)) vst<T, NC>(xs + r * NC, v);
+        }
+        if (tid < NC) {
+            int cnt = 0;
+            if (tid < nc) {
+                const uint32_t cg = c0 + tid, q = cg / dimdw;
+                const uint32_t cc = DM_IN(cg - q * dimdw, dimdw) ? cg - q * dimdw : 0u;
+                const unsigned id = a.wd[cc] & imask;
+                const T dd = a.dd[cc];
+                cnt = a.cd[cc];
+                // the bath part alone and the impurity part are added in this
+                // order per row below, as k_hxv does
+                for (int iu = 0; iu < ni; iu++)
+                    cdg[tid][iu] = a.dint[a.dswap ? id * ni + iu : iu * ni + id];
+                ndd[tid] = dd;
+            } else {
+                for (int iu = 0; iu < ni; iu++) cdg[tid][iu] = T(0);
+                ndd[tid] = T(0);
+            }
+            ncnt[tid] = min(cnt, KD);
+        }
+        for (int t = tid; t < NC * 8; t += bd) {
+            const int j = t >> 3, e = t & 7;
+            if (j < nc && e < KD) {
+                const uint32_t cg = c0 + j, q = cg / dimdw, cc = cg - q * dimdw;
+                if (e < (int)a.cd[cc] && DM_IN(e, a.W)) {
+                    const uint32_t en = a.ed[(int64_t)e * dimdw + cc];
+                    const bool ok = DM_IN(ell_par(en), a.P) && DM_IN(ell_col(en), dimdw);
+                    const T v = ok ? a.pd[ell_par(en)] : T(0);
+                    nval[j][e] = ell_neg(en) ? -v : v;
+                    noff[j][e] = ok ? (q * dimdw + ell_col(en)) * dimup : 0u;
+                }
+            }
+        }
+        __syncthreads();
+        for (uint32_t r = tid; r < dimup; r += bd) {
+            // 1. global loads: the neighbour columns' row, the hop table
+            T nb[NC][KD];
+            int cnt[NC];
+#pragma unroll
+            for (int j = 0; j < NC; j++) {
+                cnt[j] = ncnt[j];
+                uint32_t o[8];
+                const uint4 q0 = *reinterpret_cast<const uint4 *>(&noff[j][0]);
+                const uint4 q1 = *reinterpret_cast<const uint4 *>(&noff[j][4]);
+                o[0] = q0.x; o[1] = q0.y; o[2] = q0.z; o[3] = q0.w;
+                o[4] = q1.x; o[5] = q1.y; o[6] = q1.z; o[7] = q1.w;
+#pragma unroll
+                for (int e = 0; e < KD; e++) {
+                    nb[j][e] = T(0);
+                    if (e < cnt[j] && DM_IN(o[e] + r, total)) nb[j][e] = __ldcg(x + (o[e] + r));
+                }
+            }
+            uint32_t en[KU];
+#pragma unroll
+            for (int q = 0; q < KU; q++) en[q] = eux[q * dimup + r];
+            const uint32_t iu = a.wu[r] & imask;
+            const T du = a.du[r];
+            // 2. diagonal
+            T acc[NC], x0[NC];
+            vld<T, NC>(xs + r * NC, x0);
+#pragma unroll
+            for (int j = 0; j < NC; j++) acc[j] = (du + ndd[j] + cdg[j][iu]) * x0[j];
+            // 3. row hops: NC-wide gathers from the tile
+#pragma unroll
+            for (int q = 0; q < KU; q++) {
+                const T v = spv[en[q] >> 24];
+                const uint32_t bo = en[q] & 0xFFFFFFu;
+                T xg[NC];
+#pragma unroll
+                for (int j = 0; j < NC; j++) xg[j] = T(0);
+                if ((en[q] >> 24) != kLeanZero && DM_IN(bo / 16, dimup))
+                    vld<T, NC>(reinterpret_cast<const T *>(smem_raw + bo), xg);
+#pragma unroll
+                for (int j = 0; j < NC; j++) acc[j] += v * xg[j];
+            }
+            T xp[NC];
+            if (LZ) {
+#pragma unroll
+                for (int j = 0; j < NC; j++) {
+                    const uint32_t idx = (c0 + j) * dimup + r;
+                    xp[j] = j < nc && DM_IN(idx, total) ? __ldcs(xprev + idx) : T(0);
+                }
+            }
+            // 4. column hops
+#pragma unroll
+            for (int j = 0; j < NC; j++) {
+                T vv[8];
+#pragma unroll
+                for (int e = 0; e < 8; e += NC) {
+                    T t4[NC];
+                    vld<T, NC>(&nval[j][e], t4);
+#pragma unroll
+                    for (int i = 0; i < NC; i++) vv[e + i] = t4[i];
+                }
+#pragma unroll
+                for (int e = 0; e < KD; e++)
+                    if (e < cnt[j]) acc[j] += vv[e] * nb[j][e];
+            }
+            // 5. Lanczos combination, store, alpha partial
+            double part = 0.0;
+#pragma unroll
+            for (int j = 0; j < NC; j++) {
+                if (j >= nc) continue;
+                const uint32_t idx = (c0 + j) * dimup + r;
+                if (!DM_IN(idx, total)) continue;
+                if (LZ) {
+                    if constexpr (sizeof(T) == 8) {
+                        acc[j] = sc * acc[j] - cprev * xp[j];
+                    } else {
+                        T t = -cpl * xp[j];
+                        t = fmaf(-cph, xp[j], t);
+                        t = fmaf(scl, acc[j], t);
+                        acc[j] = fmaf(sch, acc[j], t);
+                    }
+                    part = fma((double)x0[j], (double)acc[j], part);
+                }
+                __stcs(y + idx, acc[j]);
+            }
+            if (LZ) dot.add(part);
+        }
+    }
+    if (MODE == 1) {
+        CSum arr[1] = {dot};
+        double tot[1];
+        if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {
+            if (tid == 0) a.alpha[a.k] = sc * tot[0];
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // k_hxv_global: the same product for sectors whose columns do not fit in
-// shared memory (DimUp x 16 bytes above the 200 KB a tile may take: Ns >= 16
-// near half filling).  One thread per element, in index order (a warp holds
+// shared memory (DimUp x 16 bytes above the 224 KB a tile may take, or above
+// 200 KB where k_hxv_lean does not serve the sector: Ns >= 17 near half filling).  One thread per element, in index order (a warp holds
 // consecutive rows of one column): the up hops gather from the element's own
 // column in global memory (a column is at most a few hundred KB, served from
 // L1/L2), the down hops read whole neighbour columns (coalesced), the tables
@@ -1031,8 +1227,26 @@ struct HxvCfg {
     int nc, vw, threads;
     size_t smem;
     int grid;
+    bool big;     // one tile per SM: k_hxv_lean with kBigThreads threads
     bool global;  // the columns do not fit in shared memory: k_hxv_global
 };
+
+// One CTA of 768 threads (80 registers) per SM for tiles of more than 200 KB:
+// Ns=16 at half filling has columns of 12,870 rows, 206 KB a tile, and its FP64
+// product takes 2.48 ms against 5.01 ms with the columns in global memory (the
+// vectors, 1.3 GB each, are 0.40 ms of HBM).
+constexpr size_t kBigTile = 224 * 1024;
+constexpr int kBigThreads = 768;
+
+// Whether the lean kernels serve this sector view with vectors of vw rows: at
+// most 8 hops per word on either side, signed coupling indices within 8 bits,
+// row offsets within 24 bits, fewer than 2^32 stacked elements.
+template <typename T>
+static bool lean_shape(const dmfted_ctx *c, const HxvArgs<T> &a, int vw) {
+    return vw == 2 && c->tune_hxv != 1 && c->tune_hxv != 2 && a.eux && a.ku_max <= 8 &&
+           a.kd_max <= 8 && 2 * a.P <= (int)kLeanZero && a.dimup * 16 < (1 << 24) &&
+           (double)a.dimup * a.dimdw * std::max(a.nstack, 1) < 4.0e9;
+}
 
 
 static bool aligned_to(const void *p, size_t b) { return ((uintptr_t)p % b) == 0; }
@@ -1051,7 +1265,11 @@ static HxvCfg hxv_config(dmfted_ctx *c, const SectorView &s, const HxvArgs<T> &a
     const int64_t ncols = a.dimdw * nstack;
     g.nc = 16 / (int)sizeof(T);  // one 16-byte gather serves the whole tile
     const size_t tile = (size_t)a.dimup * sizeof(T) * g.nc;
-    g.global = tile > (size_t)200 * 1024 || c->tune_hxv == 3;
+    // a tile above 200 KB, up to what one CTA can take beside 4 KB of tables,
+    // runs with one large CTA per SM in k_hxv_lean; otherwise the columns
+    // stay in global memory
+    g.big = tile > (size_t)200 * 1024 && tile <= kBigTile && lean_shape<T>(c, a, g.vw);
+    g.global = (tile > (size_t)200 * 1024 && !g.big) || c->tune_hxv == 3;
     if (g.global) {
         // one thread per element
         g.threads = 256;
@@ -1060,7 +1278,7 @@ static HxvCfg hxv_config(dmfted_ctx *c, const SectorView &s, const HxvArgs<T> &a
                                         std::min<int64_t>(kMaxRedBlocks, 8 * num_sms(c)));
         return g;
     }
-    g.threads = (a.dimup <= (int64_t)128 * g.vw * 2) ? 128 : 256;
+    g.threads = g.big ? kBigThreads : (a.dimup <= (int64_t)128 * g.vw * 2) ? 128 : 256;
     g.smem = tile;
     g.grid = (int)std::min<int64_t>((ncols + g.nc - 1) / g.nc, kMaxRedBlocks);
     return g;
@@ -1096,13 +1314,13 @@ static void launch_rv(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int n
     c->launches++;
 }
 
-template <typename T, int KU, int KD, int MODE, int MB>
+template <typename T, int KU, int KD, int MODE, int MB, int NT = 256>
 static void launch_lean_mb(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int nvec) {
-    auto kern = k_hxv_lean<T, KU, KD, MODE, MB>;
+    auto kern = k_hxv_lean<T, KU, KD, MODE, MB, NT>;
     static bool attr_set[64] = {false};
     if (!attr_set[c->device & 63]) {
         DM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     200 * 1024));
+                                     NT > 256 ? (int)kBigTile : 200 * 1024));
         attr_set[c->device & 63] = true;
     }
     dim3 grid(g.grid, nvec);
@@ -1116,7 +1334,8 @@ static void launch_lean_mb(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, 
 // latency hiding pays more than the registers.  DMFTED_HXV_OCC=2 keeps two.
 template <typename T, int KU, int KD, int MODE>
 static void launch_lean_k(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int nvec) {
-    if (c->tune_occ == 2) launch_lean_mb<T, KU, KD, MODE, kRvBlocks>(c, a, g, nvec);
+    if (g.big) launch_lean_mb<T, KU, KD, MODE, 1, kBigThreads>(c, a, g, nvec);
+    else if (c->tune_occ == 2) launch_lean_mb<T, KU, KD, MODE, kRvBlocks>(c, a, g, nvec);
     else launch_lean_mb<T, KU, KD, MODE, 3>(c, a, g, nvec);
 }
 
@@ -1130,14 +1349,23 @@ static void launch_lean(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int
     else launch_lean_k<T, 7, 7, MODE>(c, a, g, nvec);
 }
 
-// Whether the lean kernel serves this sector view: at most 8 hops per word
-// on either side, signed coupling indices within 8 bits, row offsets within
-// 24 bits, two-row vectors, fewer than 2^32 stacked elements.
-template <typename T>
-static bool lean_ok(const dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g) {
-    return g.vw == 2 && c->tune_hxv != 1 && c->tune_hxv != 2 && a.eux && a.ku_max <= 8 &&
-           a.kd_max <= 8 && 2 * a.P <= (int)kLeanZero && a.dimup * 16 < (1 << 24) &&
-           (double)a.dimup * a.dimdw * a.nstack < 4.0e9;
+template <typename T, int KU, int KD, int MODE>
+static void launch_lean1_k(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int nvec) {
+    auto kern = k_hxv_lean1<T, KU, KD, MODE>;
+    static bool attr_set[64] = {false};
+    if (!attr_set[c->device & 63]) {
+        DM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     200 * 1024));
+        attr_set[c->device & 63] = true;
+    }
+    kern<<<dim3(g.grid, nvec), g.threads, g.smem, c->stream>>>(a, a.eux);
+    DM_CHECK_LAUNCH();
+    c->launches++;
+}
+template <typename T, int MODE>
+static void launch_lean1(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int nvec) {
+    if (a.ku_max > 7 || a.kd_max > 7) launch_lean1_k<T, 8, 8, MODE>(c, a, g, nvec);
+    else launch_lean1_k<T, 7, 7, MODE>(c, a, g, nvec);
 }
 
 template <typename T, bool LZ>
@@ -1149,13 +1377,16 @@ static void launch_hxv(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int 
     // offsets within the stacked vector
     const bool rv = g.vw == 2 && c->tune_hxv != 1 &&
                     (double)a.dimup * a.dimdw * a.nstack < 4.0e9;
-    const bool lean = !g.global && lean_ok<T>(c, a, g);
+    const bool lean = !g.global && lean_shape<T>(c, a, g.vw);
+    // one-row vectors (odd row counts): the one-row form of the lean kernel
+    const bool lean1 = !g.global && g.vw == 1 && lean_shape<T>(c, a, 2);
     hv_timer_begin(c);
     if (g.global) {
         k_hxv_global<T, LZ><<<dim3(g.grid, nvec), g.threads, 0, c->stream>>>(a);
         DM_CHECK_LAUNCH();
         c->launches++;
     } else if (lean) launch_lean<T, LZ ? 1 : 0>(c, a, g, nvec);
+    else if (lean1) launch_lean1<T, LZ ? 1 : 0>(c, a, g, nvec);
     else if (rv) launch_rv<T, LZ>(c, a, g, nvec);
     else if (g.vw == 2) launch_nc<T, NCT, 2, LZ>(c, a, g, nvec);
     else launch_nc<T, NCT, 1, LZ>(c, a, g, nvec);
