@@ -1240,7 +1240,9 @@ int dmfted_cg_fit_batch(dmfted_ctx *c, int32_t nbatch, int32_t nbath, int32_t L,
     const size_t na = (size_t)nbatch * 2 * nbath;
     DBuf<double> buf;
     buf.alloc(na + 4 * (size_t)L + nbatch);
-    double *da = buf.p, *dx = da + na, *dg = dx + L, *dw = dg + 2 * (size_t)L, *dc = dw + L;
+    // the complex target right after the even-sized parameters: 16-byte aligned
+    // for every L
+    double *da = buf.p, *dg = da + na, *dx = dg + 2 * (size_t)L, *dw = dx + L, *dc = dw + L;
     DBuf<int> ibuf;
     ibuf.alloc(2 * (size_t)nbatch);
     DM_CUDA(cudaMemcpyAsync(da, a, na * 8, cudaMemcpyHostToDevice, c->stream));

@@ -1,11 +1,12 @@
 // H*v of a batched job with the whole vector on chip.
 //
 // A job (one sector) is run by CL CTAs of kOcThreads threads (one cluster, or
-// one CTA).  The vector is kept as a matrix whose rows are the words of the
-// spin with the smaller class and whose columns are the other spin's (H is
-// symmetric in the two factors); each CTA keeps a contiguous block of columns
-// in shared memory, with the row hop table of the sector and the column hop
-// tables of its own columns.
+// one CTA).  The vector is the DimUp x DimDw matrix; each CTA keeps a contiguous
+// block of columns in shared memory, with the row hop table of the sector and
+// the column hop tables of its own columns: a Lanczos step reads nothing from
+// L2.  Every element's arithmetic is that of the jobs in batch.cu, and the sums
+// do not depend on the split of the elements (CSum::add_product), so both give
+// the same numbers to the last digit: a bath fit's path hangs on it.
 //  * Row hops gather from the element's own column in this CTA's shared memory.
 //    A thread owns one row and walks over columns, four at a time, so that one
 //    table entry and one coupling serve four gathers.
