@@ -155,71 +155,105 @@ __global__ void k_ell_build(int ns, const ClassTab ct, int norb, int nbath, int 
 // 3432-row class of 14 sites at 7 particles this cuts the gather wavefronts
 // of the H*v by 22 % over the greedy order (5399 -> 4184 per column tile;
 // 3010 would be conflict-free).
+//
+// One warp climbs one quarter warp's rows.  The four slot costs of a trial swap
+// are computed at once, eight lanes (one row each) per cost: distinct targets and
+// quad loads by warp matches.  (One thread per quarter, its tables in local
+// memory, and one launch per class took 40 ms for the 13 classes of 12 sites;
+// one launch of these 0.4 ms, with the same tables.)
 constexpr int kClimbRows = 8, kClimbW = 16, kClimbPasses = 32;
+constexpr int kClimbWarps = 4;
 
-__device__ int climb_slot_cost(const uint32_t (&t)[kClimbRows][kClimbW], const int *self, const int *c,
-                               int m, int q) {
-    int load[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = 0; i < m; i++) {
-        const uint32_t ti = q < c[i] ? t[i][q] : (uint32_t)self[i];
-        bool dup = false;
-        for (int j = 0; j < i; j++) dup |= (q < c[j] ? t[j][q] : (uint32_t)self[j]) == ti;
-        if (!dup) load[ti & 7u]++;
-    }
-    int mx = 0, sq = 0;
-    for (int b = 0; b < 8; b++) {
-        mx = max(mx, load[b]);
-        sq += load[b] * load[b];
-    }
-    return mx * 64 + sq;
+// What the table kernels need of every class, one class per blockIdx.y.
+struct EllClasses {
+    int64_t off[kMaxNs + 1], rows[kMaxNs + 1];
+    uint8_t climb[kMaxNs + 1];
+};
+__host__ __device__ inline int ell_vw(int64_t rows) { return rows % 2 == 0 ? 2 : 1; }
+__host__ __device__ inline int64_t ell_groups(int64_t rows) {
+    const int vw = ell_vw(rows), span = vw == 2 ? 64 : 32;
+    return (rows + span - 1) / span * vw;
 }
 
-__device__ void climb_quarter(uint32_t *e, int64_t rows, const int64_t *rr, const uint8_t *cnt,
-                              int64_t off, int m) {
-    uint32_t ent[kClimbRows][kClimbW], t[kClimbRows][kClimbW];
+struct ClimbTables {
+    uint32_t t[kClimbRows][kClimbW], ent[kClimbRows][kClimbW];  // targets, entries
     int c[kClimbRows], self[kClimbRows];
-    for (int i = 0; i < m; i++) {
-        c[i] = min((int)cnt[off + rr[i]], kClimbW);
-        self[i] = (int)rr[i];
-        for (int q = 0; q < c[i]; q++) {
-            ent[i][q] = e[(int64_t)q * rows + rr[i]];
-            t[i][q] = ell_col(ent[i][q]);
+};
+
+__device__ void climb_quarter(ClimbTables &S, uint32_t *e, int64_t rows, const int64_t r0,
+                              int64_t stride, const uint8_t *cnt, int64_t off, int m) {
+    const int lane = threadIdx.x & 31, grp = lane >> 3, row = lane & 7;
+    __syncwarp();
+    for (int i = lane; i < m * kClimbW; i += 32) {
+        const int r = i / kClimbW, q = i % kClimbW;
+        const int64_t rr = r0 + r * stride;
+        const int c = min((int)cnt[off + rr], kClimbW);
+        if (q == 0) {
+            S.c[r] = c;
+            S.self[r] = (int)rr;
+        }
+        if (q < c) {
+            S.ent[r][q] = e[(int64_t)q * rows + rr];
+            S.t[r][q] = ell_col(S.ent[r][q]);
         }
     }
+    __syncwarp();
+    const int crow = row < m ? S.c[row] : 0;
     for (int pass = 0; pass < kClimbPasses; pass++) {
         bool improved = false;
-        for (int i = 0; i < m; i++)
-            for (int a = 0; a < c[i]; a++)
-                for (int b = a + 1; b < c[i]; b++) {
-                    const int before = climb_slot_cost(t, self, c, m, a) + climb_slot_cost(t, self, c, m, b);
-                    uint32_t x = t[i][a];
-                    t[i][a] = t[i][b];
-                    t[i][b] = x;
-                    const int after = climb_slot_cost(t, self, c, m, a) + climb_slot_cost(t, self, c, m, b);
-                    if (after < before) {
+        for (int i = 0; i < m; i++) {
+            const int ci = S.c[i];
+            for (int a = 0; a < ci; a++)
+                for (int b = a + 1; b < ci; b++) {
+                    // lanes 0..7: slot a, 8..15: slot b, 16..31: the same after
+                    // the swap of row i's slots a and b
+                    int q = (grp & 1) ? b : a;
+                    if (grp >= 2 && row == i) q = a + b - q;
+                    const bool act = row < m;
+                    const uint32_t ti = !act ? 0u : q < crow ? S.t[row][q] : (uint32_t)S.self[row];
+                    const unsigned same = __match_any_sync(
+                        0xffffffffu, act ? ((unsigned)grp << 20 | ti) : 0x80000000u | (unsigned)lane);
+                    const bool first = act && __ffs(same) - 1 == lane;
+                    const unsigned quad = __match_any_sync(
+                        0xffffffffu, first ? ((unsigned)grp << 3 | (ti & 7u)) : 0x100u | (unsigned)lane);
+                    int mx = first ? __popc(quad) : 0, sq = mx;
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) {
+                        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                        sq += __shfl_xor_sync(0xffffffffu, sq, o);
+                    }
+                    int cost = mx * 64 + sq;
+                    cost += __shfl_xor_sync(0xffffffffu, cost, 8);  // both slots
+                    if (__shfl_sync(0xffffffffu, cost, 16) < __shfl_sync(0xffffffffu, cost, 0)) {
                         improved = true;
-                        x = ent[i][a];
-                        ent[i][a] = ent[i][b];
-                        ent[i][b] = x;
-                    } else {
-                        x = t[i][a];
-                        t[i][a] = t[i][b];
-                        t[i][b] = x;
+                        __syncwarp();
+                        if (lane == 0) {
+                            uint32_t x = S.t[i][a];
+                            S.t[i][a] = S.t[i][b];
+                            S.t[i][b] = x;
+                            x = S.ent[i][a];
+                            S.ent[i][a] = S.ent[i][b];
+                            S.ent[i][b] = x;
+                        }
+                        __syncwarp();
                     }
                 }
+        }
         if (!improved) break;
     }
-    for (int i = 0; i < m; i++)
-        for (int q = 0; q < c[i]; q++) e[(int64_t)q * rows + rr[i]] = ent[i][q];
+    for (int i = lane; i < m * kClimbW; i += 32) {
+        const int r = i / kClimbW, q = i % kClimbW;
+        if (q < S.c[r]) e[(int64_t)q * rows + r0 + r * stride] = S.ent[r][q];
+    }
 }
 
-__global__ void k_ell_balance(int ns, int n, int64_t off, int W, int vw, int gsize,
-                              const uint8_t *cnt, uint32_t *ell) {
-    const int64_t rows = binom_d(ns, n);
+__global__ void k_ell_balance(const EllClasses cl, int W, int gsize, const uint8_t *cnt,
+                              uint32_t *ell) {
+    const int64_t rows = cl.rows[blockIdx.y], off = cl.off[blockIdx.y];
+    const int vw = ell_vw(rows);
     const int64_t span = vw == 2 ? 64 : 32;
-    const int64_t ngroups = ((rows + span - 1) / span) * vw;
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (g >= ngroups) return;
+    if (g >= ell_groups(rows)) return;
     const int64_t blk = g / vw, par = g % vw;
     uint32_t *e = ell + (int64_t)W * off;
     int load[kMaxW][8];
@@ -253,35 +287,33 @@ __global__ void k_ell_balance(int ns, int n, int64_t off, int W, int vw, int gsi
     }
 }
 
-// The hill climbing of k_ell_balance's groups, one thread per quarter warp
-// (launched after the greedy pass, in classes whose words have at most 8
+// The hill climbing of k_ell_balance's groups, one warp per quarter warp
+// (launched after the greedy pass, for the classes whose words have at most 8
 // hops, with gsize 8 and at most kClimbW hops per word).
-__global__ void k_ell_climb(int ns, int n, int64_t off, int W, int vw, const uint8_t *cnt,
-                            uint32_t *ell) {
-    const int64_t rows = binom_d(ns, n);
+__global__ void __launch_bounds__(32 * kClimbWarps) k_ell_climb(const EllClasses cl, int W,
+                                                                 const uint8_t *cnt, uint32_t *ell) {
+    __shared__ ClimbTables tabs[kClimbWarps];
+    if (!cl.climb[blockIdx.y]) return;
+    const int64_t rows = cl.rows[blockIdx.y], off = cl.off[blockIdx.y];
+    const int vw = ell_vw(rows);
     const int64_t span = vw == 2 ? 64 : 32;
-    const int64_t nq = ((rows + span - 1) / span) * vw * 4;
-    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (g >= nq) return;
+    const int64_t g = blockIdx.x * (int64_t)kClimbWarps + (threadIdx.x >> 5);
+    if (g >= ell_groups(rows) * 4) return;
     const int64_t grp = g / 4, blk = grp / vw, par = grp % vw;
-    const int l0 = (int)(g % 4) * kClimbRows;
-    uint32_t *e = ell + (int64_t)W * off;
-    int64_t rr[kClimbRows];
-    int m = 0;
-    for (int i = 0; i < kClimbRows; i++) {
-        const int64_t r = blk * span + (int64_t)(l0 + i) * vw + par;
-        if (r < rows) rr[m++] = r;
-    }
-    if (m > 1) climb_quarter(e, rows, rr, cnt, off, m);
+    const int64_t r0 = blk * span + (g % 4) * kClimbRows * vw + par;
+    const int64_t m = r0 < rows ? min((int64_t)kClimbRows, (rows - 1 - r0) / vw + 1) : 0;
+    if (m > 1)
+        climb_quarter(tabs[threadIdx.x >> 5], ell + (int64_t)W * off, rows, r0, vw, cnt, off, (int)m);
 }
 
-// Lean gather table of one class from its balanced ELL table (same slot
+// Lean gather table of every class from its balanced ELL table (same slot
 // order): hop e of row r becomes (target row * 16) | (2 * coupling + sign) << 24;
 // slots at or beyond the row's hop count become zero-coupling entries that
 // point at the row itself (conflict-free: the rows of a quarter warp sit in
 // distinct bank quads).
-__global__ void k_ellx_build(int64_t rows, int64_t off, int W, int WX, const uint8_t *cnt,
+__global__ void k_ellx_build(const EllClasses cl, int W, int WX, const uint8_t *cnt,
                              const uint32_t *ell, uint32_t *ellx) {
+    const int64_t rows = cl.rows[blockIdx.y], off = cl.off[blockIdx.y];
     const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (r >= rows) return;
     const int c = cnt[off + r];
@@ -462,30 +494,36 @@ void fock_set_couplings(dmfted_ctx *c) {
                 for (int64_t r = 0; r < c->binom[n]; r++)
                     t.cls_max[n] = std::max<int>(t.cls_max[n], hc[c->class_poff[n] + r]);
         }
-        // gather grouping of the H*v: two rows per thread for even class sizes
-        for (int n = 0; rebuild && n <= c->ns; n++) {
-            const int vw = (c->binom[n] % 2 == 0) ? 2 : 1;
-            const int64_t ng = ((c->binom[n] + (vw == 2 ? 63 : 31)) / (vw == 2 ? 64 : 32)) * vw;
+        // gather order of the H*v (two rows per thread for even class sizes),
+        // every class in one launch: the classes do not depend on one another
+        if (rebuild) {
+            EllClasses cl{};
             const int gsize = c->tune_ell_group > 0 ? c->tune_ell_group : 8;
-            k_ell_balance<<<div_up(ng, 64), 64, 0, c->stream>>>(
-                c->ns, n, c->class_poff[n], std::max(c->W, 1), vw, gsize, t.cnt.p, t.ell.p);
+            int64_t rmax = 1, gmax = 1;
+            bool any = false;
+            for (int n = 0; n <= c->ns; n++) {
+                cl.off[n] = c->class_poff[n];
+                cl.rows[n] = c->binom[n];
+                cl.climb[n] = t.cls_max[n] <= 8 && gsize == kClimbRows && std::max(c->W, 1) <= kClimbW;
+                any = any || cl.climb[n];
+                rmax = std::max(rmax, cl.rows[n]);
+                gmax = std::max(gmax, ell_groups(cl.rows[n]));
+            }
+            const unsigned ncl = (unsigned)c->ns + 1;
+            k_ell_balance<<<dim3(div_up(gmax, 64), ncl), 64, 0, c->stream>>>(
+                cl, std::max(c->W, 1), gsize, t.cnt.p, t.ell.p);
             DM_CHECK_LAUNCH();
             c->launches++;
-            if (t.cls_max[n] <= 8 && gsize == kClimbRows && std::max(c->W, 1) <= kClimbW) {
-                k_ell_climb<<<div_up(ng * 4, 64), 64, 0, c->stream>>>(
-                    c->ns, n, c->class_poff[n], std::max(c->W, 1), vw, t.cnt.p, t.ell.p);
+            if (any) {
+                k_ell_climb<<<dim3(div_up(gmax * 4, kClimbWarps), ncl), 32 * kClimbWarps, 0,
+                              c->stream>>>(cl, std::max(c->W, 1), t.cnt.p, t.ell.p);
                 DM_CHECK_LAUNCH();
                 c->launches++;
             }
-        }
-        if (rebuild) {
-            for (int n = 0; n <= c->ns; n++) {
-                k_ellx_build<<<div_up(c->binom[n], 256), 256, 0, c->stream>>>(
-                    c->binom[n], c->class_poff[n], std::max(c->W, 1), c->WX, t.cnt.p, t.ell.p,
-                    t.ellx.p);
-                DM_CHECK_LAUNCH();
-                c->launches++;
-            }
+            k_ellx_build<<<dim3(div_up(rmax, 256), ncl), 256, 0, c->stream>>>(
+                cl, std::max(c->W, 1), c->WX, t.cnt.p, t.ell.p, t.ellx.p);
+            DM_CHECK_LAUNCH();
+            c->launches++;
         }
         c->ell_pattern[s] = pattern;
     }
