@@ -188,12 +188,50 @@ __global__ void k_interleave_split(const double *z, double *re, double *im, int6
         im[i] = z[2 * i + 1];
     }
 }
+// The same with the complex side in pinned host memory, whole complex numbers
+// per access.
+__global__ void __launch_bounds__(256) k_stage_in(const double2 *z, double *re, double *im, int64_t n) {
+    pdl_begin();
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const double2 v = z[i];
+        re[i] = v.x;
+        im[i] = v.y;
+    }
+}
+__global__ void __launch_bounds__(256) k_stage_out(const double *re, const double *im, double2 *z,
+                                                   int64_t n) {
+    pdl_begin();
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+        z[i] = make_double2(re[i], im[i]);
+}
 __global__ void k_interleave_join(const double *re, const double *im, double *z, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         z[2 * i] = re[i];
         z[2 * i + 1] = im ? im[i] : 0.0;
     }
+}
+
+// The context's pinned staging buffer with room for n doubles; false when the
+// host will not pin it (the caller copies as for large vectors).
+// Through the Python call, against driver copies: 400 states 25.5 and 41.0 us,
+// 4,900 states 39 and 53, 15,876 states 59 and 77; at 44,100 (126 us) the two are
+// even.
+constexpr int64_t kStageMax = 1 << 14;
+static bool stage_ready(dmfted_ctx *c, size_t n) {
+    if (c->hstage_n >= n) return true;
+    if (c->hstage) cudaFreeHost(c->hstage);
+    c->hstage = nullptr;
+    c->hstage_n = 0;
+    if (cudaMallocHost(reinterpret_cast<void **>(&c->hstage), n * sizeof(double)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->hstage = nullptr;
+        return false;
+    }
+    c->hstage_n = n;
+    return true;
 }
 
 static int ew(dmfted_ctx *c, int64_t n) {
@@ -696,6 +734,7 @@ int dmfted_free(dmfted_ctx *c) {
     }
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
+    if (c->hstage) cudaFreeHost(c->hstage);
     delete c;
     if (st) cudaStreamDestroy(st);
     if (st2) cudaStreamDestroy(st2);
@@ -797,15 +836,29 @@ int dmfted_hxv_c128(dmfted_ctx *c, int32_t nloc, const double *v, double *hv) {
     const int64_t n = s.dim;
     c->wv64.alloc(6 * n);
     double *z = c->wv64.p, *x = z + 2 * n, *y = x + 2 * n;
-    DM_CUDA(cudaMemcpyAsync(z, v, 2 * n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    k_interleave_split<<<ew(c, n), 256, 0, c->stream>>>(z, x, x + n, n);
-    DM_CHECK_LAUNCH();
-    hxv_f64(c, s, x, y, 2);
-    k_interleave_join<<<ew(c, n), 256, 0, c->stream>>>(y, y + n, z, n);
-    DM_CHECK_LAUNCH();
-    c->launches += 2;
-    DM_CUDA(cudaMemcpyAsync(hv, z, 2 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    DM_CUDA(cudaStreamSynchronize(c->stream));
+    // small vectors: two copies on the host and kernels that reach over to the
+    // pinned buffer, instead of two staged driver copies
+    if (n <= kStageMax && stage_ready(c, 4 * (size_t)n)) {
+        double *in = c->hstage, *out = in + 2 * n;
+        std::memcpy(in, v, 2 * n * sizeof(double));
+        launch_overlapped(c, k_stage_in, dim3((unsigned)ew(c, n)), 256, 0,
+                          reinterpret_cast<const double2 *>(in), x, x + n, n);
+        hxv_f64(c, s, x, y, 2);
+        launch_overlapped(c, k_stage_out, dim3((unsigned)ew(c, n)), 256, 0, (const double *)y,
+                          (const double *)(y + n), reinterpret_cast<double2 *>(out), n);
+        DM_CUDA(cudaStreamSynchronize(c->stream));
+        std::memcpy(hv, out, 2 * n * sizeof(double));
+    } else {
+        DM_CUDA(cudaMemcpyAsync(z, v, 2 * n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        k_interleave_split<<<ew(c, n), 256, 0, c->stream>>>(z, x, x + n, n);
+        DM_CHECK_LAUNCH();
+        hxv_f64(c, s, x, y, 2);
+        k_interleave_join<<<ew(c, n), 256, 0, c->stream>>>(y, y + n, z, n);
+        DM_CHECK_LAUNCH();
+        c->launches += 2;
+        DM_CUDA(cudaMemcpyAsync(hv, z, 2 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        DM_CUDA(cudaStreamSynchronize(c->stream));
+    }
     API_END
 }
 

@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(256, kHxvMinBlocks) k_hxv(const HxvArgs<T> a) 
     __shared__ T sval[NC][kMaxW];
     __shared__ int64_t soff[NC][kMaxW];
 
+    pdl_begin();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
     }
@@ -365,6 +366,7 @@ __global__ void __launch_bounds__(256, kRvBlocks) k_hxv_rv(const HxvArgs<T> a) {
     __shared__ __align__(16) T nval[NC][kMaxW];
     __shared__ int scnt[NC];
 
+    pdl_begin();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
     }
@@ -667,6 +669,7 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
     __shared__ __align__(16) uint32_t noff[NC][8];
     __shared__ __align__(16) T nval[NC][8];
 
+    pdl_begin();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
     }
@@ -920,6 +923,7 @@ __global__ void __launch_bounds__(256, 4) k_hxv_lean1(const HxvArgs<T> a,
     __shared__ T ndd[NC];
     __shared__ int ncnt[NC];
 
+    pdl_begin();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
     }
@@ -1284,6 +1288,22 @@ static HxvCfg hxv_config(dmfted_ctx *c, const SectorView &s, const HxvArgs<T> &a
     return g;
 }
 
+// Lanczos steps, and plain products of at most a CTA per SM, overlap the end of
+// the stream's previous kernel (a step of Ns=12 24 -> 21 us); larger plain
+// products back to back lose 1 % by it (CTAs that wait hold the SMs' slots).
+template <bool LZ, typename... KArgs, typename... Args>
+static void launch_product(dmfted_ctx *c, void (*kern)(KArgs...), const HxvCfg &g, int nvec,
+                           Args &&...args) {
+    const dim3 grid(g.grid, nvec);
+    if (LZ || (int64_t)g.grid * nvec <= num_sms(c)) {
+        launch_overlapped(c, kern, grid, g.threads, g.smem, args...);
+        return;
+    }
+    kern<<<grid, g.threads, g.smem, c->stream>>>(args...);
+    DM_CHECK_LAUNCH();
+    c->launches++;
+}
+
 template <typename T, int NC, int VW, bool LZ>
 static void launch_nc(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int nvec) {
     auto kern = k_hxv<T, NC, VW, LZ>;
@@ -1293,10 +1313,7 @@ static void launch_nc(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int n
                                      200 * 1024));
         attr_set[c->device & 63] = true;
     }
-    dim3 grid(g.grid, nvec);
-    kern<<<grid, g.threads, g.smem, c->stream>>>(a);
-    DM_CHECK_LAUNCH();
-    c->launches++;
+    launch_product<LZ>(c, kern, g, nvec, a);
 }
 
 template <typename T, bool LZ>
@@ -1308,10 +1325,7 @@ static void launch_rv(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int n
                                      200 * 1024));
         attr_set[c->device & 63] = true;
     }
-    dim3 grid(g.grid, nvec);
-    kern<<<grid, g.threads, g.smem, c->stream>>>(a);
-    DM_CHECK_LAUNCH();
-    c->launches++;
+    launch_product<LZ>(c, kern, g, nvec, a);
 }
 
 template <typename T, int KU, int KD, int MODE, int MB, int NT = 256>
@@ -1323,10 +1337,7 @@ static void launch_lean_mb(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, 
                                      NT > 256 ? (int)kBigTile : 200 * 1024));
         attr_set[c->device & 63] = true;
     }
-    dim3 grid(g.grid, nvec);
-    kern<<<grid, g.threads, g.smem, c->stream>>>(a, a.eux);
-    DM_CHECK_LAUNCH();
-    c->launches++;
+    launch_product<MODE != 0>(c, kern, g, nvec, a, a.eux);
 }
 
 // Three CTAs per SM (register cap 80, a few bytes of spills) measured 5-9 %
@@ -1358,9 +1369,7 @@ static void launch_lean1_k(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, 
                                      200 * 1024));
         attr_set[c->device & 63] = true;
     }
-    kern<<<dim3(g.grid, nvec), g.threads, g.smem, c->stream>>>(a, a.eux);
-    DM_CHECK_LAUNCH();
-    c->launches++;
+    launch_product<MODE != 0>(c, kern, g, nvec, a, a.eux);
 }
 template <typename T, int MODE>
 static void launch_lean1(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int nvec) {

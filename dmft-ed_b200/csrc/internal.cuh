@@ -224,6 +224,11 @@ struct dmfted_ctx {
     dmfted::DBuf<double> lz_d;           // Lanczos scalar slots
     dmfted::DBuf<int> lz_s;              // Lanczos status slots
     dmfted::DBuf<double> coefb;          // Ritz coefficients
+    // pinned host staging of the procedure-pointer H*v for small vectors: the
+    // product's kernels read and write it directly (at most 2 x 16 bytes x
+    // kStageMax; freed with the context)
+    double *hstage = nullptr;
+    size_t hstage_n = 0;
     // current sector of the procedure-pointer H*v
     int cur_sector = 0;
     // work vectors (grown on demand)
@@ -517,5 +522,34 @@ void weiss_diag_device(dmfted_ctx *c, int L, int scheme, const double *hloc_aa, 
 // ---- small helpers ------------------------------------------------------------
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 int num_sms(dmfted_ctx *c);
+
+// ---- launches that overlap the end of the stream's previous kernel ----------
+// A kernel launched by launch_overlapped starts when every CTA of the previous
+// kernel in the stream has begun (its launch latency and its scheduling run under
+// that kernel's last wave) and calls pdl_begin() before it touches memory, which
+// returns once the previous kernel has completed and its writes are visible.  A
+// previous kernel that does not trigger, or another operation in between, makes
+// it an ordinary launch.
+__device__ __forceinline__ void pdl_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... KArgs, typename... Args>
+inline void launch_overlapped(dmfted_ctx *c, void (*kern)(KArgs...), dim3 grid, int threads,
+                              size_t smem, Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    DM_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+    c->launches++;
+}
 
 }  // namespace dmfted

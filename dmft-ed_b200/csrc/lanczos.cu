@@ -54,6 +54,7 @@ template <typename T, int VW>
 __global__ void __launch_bounds__(kRedThreads) k_lz_update(T *u, const T *scur, int64_t n,
                                                            LanczosScalars lz, int k, double thr,
                                                            double *partials, unsigned *counter) {
+    pdl_begin();
     if (lz.status[ST_DONE]) return;
     const double coef = lz.alpha[k] * lz.scale[k];
     CSum s;
@@ -290,13 +291,11 @@ static void launch_lz_update(dmfted_ctx *c, T *u, const T *scur, int64_t n, cons
     constexpr int VW = 16 / sizeof(T);
     const bool vec = (n % VW == 0) && ((uintptr_t)u % 16 == 0) && ((uintptr_t)scur % 16 == 0);
     if (vec)
-        k_lz_update<T, VW><<<red_grid(c, n / VW), kRedThreads, 0, c->stream>>>(
-            u, scur, n, lz, k, thr, c->red_partials.p, c->red_counter.p);
+        launch_overlapped(c, k_lz_update<T, VW>, dim3(red_grid(c, n / VW)), kRedThreads, 0, u, scur,
+                          n, lz, k, thr, c->red_partials.p, c->red_counter.p);
     else
-        k_lz_update<T, 1><<<red_grid(c, n), kRedThreads, 0, c->stream>>>(
-            u, scur, n, lz, k, thr, c->red_partials.p, c->red_counter.p);
-    DM_CHECK_LAUNCH();
-    c->launches++;
+        launch_overlapped(c, k_lz_update<T, 1>, dim3(red_grid(c, n)), kRedThreads, 0, u, scur, n, lz,
+                          k, thr, c->red_partials.p, c->red_counter.p);
 }
 
 static int ew_grid(dmfted_ctx *c, int64_t n) {
@@ -635,13 +634,11 @@ void lanczos_chain_fixed(dmfted_ctx *c, const SectorView &s, const double *v0, d
         hxv_lanczos_step_scratch<double>(c, s, Q, P, P, lz, k, partials, counter);
         const bool vec = (dim % 2 == 0) && ((uintptr_t)P % 16 == 0) && ((uintptr_t)Q % 16 == 0);
         if (vec)
-            k_lz_update<double, 2><<<red_grid(c, dim / 2), kRedThreads, 0, c->stream>>>(
-                P, Q, dim, lz, k, c->p.lanc_gf_threshold, partials, counter);
+            launch_overlapped(c, k_lz_update<double, 2>, dim3(red_grid(c, dim / 2)), kRedThreads, 0, P,
+                              Q, dim, lz, k, c->p.lanc_gf_threshold, partials, counter);
         else
-            k_lz_update<double, 1><<<rg, kRedThreads, 0, c->stream>>>(
-                P, Q, dim, lz, k, c->p.lanc_gf_threshold, partials, counter);
-        DM_CHECK_LAUNCH();
-        c->launches++;
+            launch_overlapped(c, k_lz_update<double, 1>, dim3(rg), kRedThreads, 0, P, Q, dim, lz, k,
+                              c->p.lanc_gf_threshold, partials, counter);
         std::swap(P, Q);
     }
 }
