@@ -681,6 +681,9 @@ int dmfted_init(const dmfted_params *p, const double *hloc, dmfted_ctx **out) {
         DM_CUDA(cudaMemsetAsync(c->red_counter.p, 0, 8 * sizeof(unsigned), c->stream));
         if (c->chain_lanes >= 2) {
             DM_CUDA(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));
+            DM_CUDA(cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking));
+            DM_CUDA(cudaEventCreateWithFlags(&c->ev_fork3, cudaEventDisableTiming));
+            DM_CUDA(cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming));
             DM_CUDA(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
             DM_CUDA(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
             c->red_partials2.alloc((size_t)2 * 64 * kMaxRedBlocks);
@@ -726,7 +729,8 @@ int dmfted_free(dmfted_ctx *c) {
     // here rather than left for the next context to trip over
     cudaError_t pending = c->stream ? cudaStreamSynchronize(c->stream) : cudaSuccess;
     if (c->stream2 && pending == cudaSuccess) pending = cudaStreamSynchronize(c->stream2);
-    cudaStream_t st = c->stream, st2 = c->stream2;
+    if (c->stream3 && pending == cudaSuccess) pending = cudaStreamSynchronize(c->stream3);
+    cudaStream_t st = c->stream, st2 = c->stream2, st3 = c->stream3;
     for (cudaEvent_t e : c->hv_ev_free) cudaEventDestroy(e);
     for (auto &pr : c->hv_ev) {
         cudaEventDestroy(pr.first);
@@ -734,10 +738,13 @@ int dmfted_free(dmfted_ctx *c) {
     }
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
+    if (c->ev_fork3) cudaEventDestroy(c->ev_fork3);
+    if (c->ev_join3) cudaEventDestroy(c->ev_join3);
     if (c->hstage) cudaFreeHost(c->hstage);
     delete c;
     if (st) cudaStreamDestroy(st);
     if (st2) cudaStreamDestroy(st2);
+    if (st3) cudaStreamDestroy(st3);
     DM_REQUIRE(pending == cudaSuccess, DMFTED_ERR_CUDA,
                std::string("device error pending at free: ") + cudaGetErrorString(pending));
     API_END

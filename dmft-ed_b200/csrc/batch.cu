@@ -974,7 +974,7 @@ static void run_batch_eigs(dmfted_ctx *c, int j0, int nbig, int j1, int wave, do
                       batch_tables<T>(c), reinterpret_cast<const EigsJob *>(c->bjobs.p) + j0, nbig,
                       j1 - j0, reinterpret_cast<unsigned *>(c->bint.p) + 2 * wave,
                       reinterpret_cast<T *>(c->bwork.p), c->bvec.p, c->baux.p, c->bscal.p,
-                      c->bint.p + 2 * kMaxWaves, tol, std::max(1, c->p.lanc_ncheck),
+                      c->bint.p + 4 * kMaxWaves, tol, std::max(1, c->p.lanc_ncheck),
                       BatchCaps{(int64_t)(c->bwork.n / sizeof(T)), (int64_t)c->bvec.n,
                                 (int64_t)c->baux.n, 0, (int64_t)(c->bscal.n / kEigsMaxEigen),
                                 (int64_t)c->lockpool.n},
@@ -1071,10 +1071,10 @@ static void batch_eigs_cl(dmfted_ctx *c, const std::vector<int> &list,
     c->baux.alloc(aux);
     c->bjobs.alloc(nj * sizeof(EigsJob));
     c->bscal.alloc((size_t)nj * kEigsMaxEigen);
-    c->bint.alloc(2 * kMaxWaves + nj);
+    c->bint.alloc(4 * kMaxWaves + nj);
     DM_CUDA(cudaMemcpyAsync(c->bjobs.p, q.data(), nj * sizeof(EigsJob), cudaMemcpyHostToDevice,
                             c->stream));
-    DM_CUDA(cudaMemsetAsync(c->bint.p, 0, 2 * kMaxWaves * sizeof(int), c->stream));
+    DM_CUDA(cudaMemsetAsync(c->bint.p, 0, 4 * kMaxWaves * sizeof(int), c->stream));
     const double tol = fp64 ? p.lanc_tolerance : std::max(p.lanc_tolerance, c->mixed_tol32);
     for (size_t w = 0; w < wave_end.size(); w++) {
         const int j0 = w == 0 ? 0 : wave_end[w - 1], j1 = wave_end[w];
@@ -1082,14 +1082,37 @@ static void batch_eigs_cl(dmfted_ctx *c, const std::vector<int> &list,
         while (CL > 1 && j0 + nbig < j1 &&
                c->binom[q[j0 + nbig].nup] * c->binom[q[j0 + nbig].ndw] >= c->batch_cluster_min * CL)
             nbig++;
-        if (fp64) run_batch_eigs_cl<double>(c, CL, j0, nbig, j1, (int)w, tol);
-        else run_batch_eigs_cl<float>(c, CL, j0, nbig, j1, (int)w, tol);
+        auto run = [&](int cl, int a, int big, int b, int wave) {
+            if (fp64) run_batch_eigs_cl<double>(c, cl, a, big, b, wave, tol);
+            else run_batch_eigs_cl<float>(c, cl, a, big, b, wave, tol);
+        };
+        // Clusters of 16 leave SMs idle (at most seven or eight fit the GPCs): the
+        // sectors of one CTA each start there at once, on the third stream with
+        // their own queue, instead of after the clusters' (thermal Ns=10 solve:
+        // FIGURES).
+        if (CL >= 16 && nbig > 0 && j0 + nbig < j1 && c->stream3) {
+            DM_CUDA(cudaEventRecord(c->ev_fork3, c->stream));
+            DM_CUDA(cudaStreamWaitEvent(c->stream3, c->ev_fork3, 0));
+            run(CL, j0, nbig, j0 + nbig, (int)w);
+            std::swap(c->stream, c->stream3);
+            try {
+                run(1, j0 + nbig, 0, j1, kMaxWaves + (int)w);
+            } catch (...) {
+                std::swap(c->stream, c->stream3);
+                throw;
+            }
+            std::swap(c->stream, c->stream3);
+            DM_CUDA(cudaEventRecord(c->ev_join3, c->stream3));
+            DM_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join3, 0));
+        } else {
+            run(CL, j0, nbig, j1, (int)w);
+        }
     }
     std::vector<double> ev((size_t)nj * kEigsMaxEigen);
     std::vector<int> steps(nj);
     DM_CUDA(cudaMemcpyAsync(ev.data(), c->bscal.p, ev.size() * sizeof(double),
                             cudaMemcpyDeviceToHost, c->stream));
-    DM_CUDA(cudaMemcpyAsync(steps.data(), c->bint.p + 2 * kMaxWaves, nj * sizeof(int),
+    DM_CUDA(cudaMemcpyAsync(steps.data(), c->bint.p + 4 * kMaxWaves, nj * sizeof(int),
                             cudaMemcpyDeviceToHost, c->stream));
     DM_CUDA(cudaStreamSynchronize(c->stream));
     for (int j = 0; j < nj; j++) {

@@ -214,6 +214,10 @@ struct dmfted_ctx {
     // (batch.cu, SecondLane)
     cudaStream_t stream2 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // third stream: the batched eigensolves of one CTA each beside those of a
+    // large cluster (batch.cu)
+    cudaStream_t stream3 = nullptr;
+    cudaEvent_t ev_fork3 = nullptr, ev_join3 = nullptr;
     dmfted::DBuf<double> red_partials2;
     dmfted::DBuf<unsigned> red_counter2;
     dmfted::DBuf<uint8_t> chainbuf2;
