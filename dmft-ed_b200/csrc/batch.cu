@@ -1088,8 +1088,8 @@ static void batch_eigs_cl(dmfted_ctx *c, const std::vector<int> &list,
         };
         // Clusters of 16 leave SMs idle (at most seven or eight fit the GPCs): the
         // sectors of one CTA each start there at once, on the third stream with
-        // their own queue, instead of after the clusters' (thermal Ns=10 solve:
-        // FIGURES).
+        // their own queue, instead of after the clusters' (the eigensolve
+        // phase of the Ns=10 finite-temperature solve: 23.3 -> 20.3 ms).
         if (CL >= 16 && nbig > 0 && j0 + nbig < j1 && c->stream3) {
             DM_CUDA(cudaEventRecord(c->ev_fork3, c->stream));
             DM_CUDA(cudaStreamWaitEvent(c->stream3, c->ev_fork3, 0));

@@ -117,13 +117,15 @@ __global__ void __launch_bounds__(kChi2Threads, NB <= 4 ? 6 : NB <= 8 ? 5 : NB <
         for (int t = 0; t < kChi2Threads; t += 32) s.add(sums[q][t + lane]);
         warp_reduce(s);
         if (lane == 0) {
-            const double val = s.value();
             if (q == 0) {
-                chi2[blockIdx.x] = val;
+                chi2[blockIdx.x] = s.value();
             } else if (grad) {
-                const int k = (q - 1) % NB;
-                const double v = pv[k];
-                grad[(int64_t)blockIdx.x * 2 * NB + (q - 1)] = (q <= NB ? -2.0 * v * v : -4.0 * v) * val;
+                // -2 V^2 or -4 V times the sum, rounded once (V^2 = f + fl exactly)
+                const double v = pv[(q - 1) % NB];
+                const double f = q <= NB ? v * v : 2.0 * v, fl = q <= NB ? fma(v, v, -f) : 0.0;
+                const double p = s.hi * f;
+                const double pl = fma(s.hi, f, -p) + fma(s.hi, fl, s.lo * f);
+                grad[(int64_t)blockIdx.x * 2 * NB + (q - 1)] = -2.0 * (p + pl);
             }
         }
     }
