@@ -15,9 +15,13 @@
 // it replaces, without a branch between the NB chains.  The sums are folded
 // compensated, one warp per sum, in a fixed order.  What bounds it: the FP64
 // pipe's latency at four or five CTAs per SM.  4096 sets of 9 levels, 1000
-// points: 69 us against 133 us with the sums in shared memory and divisions
-// (errors against 64-bit references alike, 2e-16 of the norm); the 19 FP64
-// operations per level and point are 40 us of the pipe.
+// points: 72 us against 133 us with the sums in shared memory and divisions; the
+// 20 FP64 operations per level and point are 42 us of the pipe.  Largest errors
+// against 64-bit references over 24 inputs, of the norm: chi^2 2.9e-16 (3.5e-16
+// before), gradient 3.49e-16 (3.53e-16); means 2.07e-16 (2.04e-16) and 2.30e-16
+// (2.22e-16).  Every accumulation is one rounded product sum and one addition: a
+// gradient term folded in by two chained fma is 2 us faster, with errors of 3.53e-16
+// and 2.33e-16.
 #include <algorithm>
 
 #include "internal.cuh"
@@ -99,7 +103,7 @@ __global__ void __launch_bounds__(kChi2Threads, NB <= 4 ? 6 : NB <= 8 ? 5 : NB <
             const double t = fma(Wr, re, Wi * im);  // Re(conj(R) r) / W
             const double u = fma(Wi, re, -Wr * im);
             sv[k] += t;
-            se[k] = fma(t, re, fma(u, im, se[k]));  // Re(conj(R) r^2) / W
+            se[k] += fma(t, re, u * im);  // Re(conj(R) r^2) / W
         }
     }
     sums[0][tid] = s0;
