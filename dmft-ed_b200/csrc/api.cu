@@ -681,9 +681,6 @@ int dmfted_init(const dmfted_params *p, const double *hloc, dmfted_ctx **out) {
         DM_CUDA(cudaMemsetAsync(c->red_counter.p, 0, 8 * sizeof(unsigned), c->stream));
         if (c->chain_lanes >= 2) {
             DM_CUDA(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));
-            DM_CUDA(cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking));
-            DM_CUDA(cudaEventCreateWithFlags(&c->ev_fork3, cudaEventDisableTiming));
-            DM_CUDA(cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming));
             DM_CUDA(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
             DM_CUDA(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
             c->red_partials2.alloc((size_t)2 * 64 * kMaxRedBlocks);

@@ -1090,7 +1090,10 @@ static void batch_eigs_cl(dmfted_ctx *c, const std::vector<int> &list,
         // sectors of one CTA each start there at once, on the third stream with
         // their own queue, instead of after the clusters' (the eigensolve
         // phase of the Ns=10 finite-temperature solve: 23.3 -> 20.3 ms).
-        if (CL >= 16 && nbig > 0 && j0 + nbig < j1 && c->stream3) {
+        if (CL >= 16 && nbig > 0 && j0 + nbig < j1 && c->stream2) {
+            if (!c->ev_fork3) DM_CUDA(cudaEventCreateWithFlags(&c->ev_fork3, cudaEventDisableTiming));
+            if (!c->ev_join3) DM_CUDA(cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming));
+            if (!c->stream3) DM_CUDA(cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking));
             DM_CUDA(cudaEventRecord(c->ev_fork3, c->stream));
             DM_CUDA(cudaStreamWaitEvent(c->stream3, c->ev_fork3, 0));
             run(CL, j0, nbig, j0 + nbig, (int)w);
