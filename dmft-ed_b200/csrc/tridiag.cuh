@@ -42,12 +42,18 @@ __device__ inline int sturm_count(const double *a, const double *b, int n, doubl
 // Sturm count: number of eigenvalues of the n x n tridiagonal (a, b[1..n-1])
 // below x, as sign changes of the leading principal minors
 //   p_i = (a_i - x) p_{i-1} - b_i^2 p_{i-2},
-// a zero pivot ratio |p_i / p_{i-1}| < pivmin counting as a negative one.  The
-// minors are rescaled by a power of two every eight steps.  Two FP64 operations,
-// a compare and a select per step (45 cycles) against the 320 of the division in
-// sturm_count; the two agree unless x is within rounding of an eigenvalue.
-__device__ inline int sturm_count_fast(const double *a, const double *b, int n, double x, double pivmin) {
-    double pp = 1.0, p = a[0] - x;
+// a zero pivot ratio |p_i / p_{i-1}| < pivmin counting as a negative one.  T, x
+// and pivmin are multiplied by s, a power of two that brings |T| near one
+// (tridiag_scale), and the minors rescaled by a power of two every eight steps:
+// eight pivots, even all at pivmin, then stay within the range of FP64 at every
+// energy unit (unscaled, eight steps of |T| = 1e-38 underflow to a wrong count),
+// and both scalings are exact.  Two FP64 operations, a compare and a select per
+// step (45 cycles) against the 320 of the division in sturm_count; the two agree
+// unless x is within rounding of an eigenvalue.
+__device__ inline int sturm_count_fast(const double *a, const double *b, int n, double x,
+                                       double pivmin, double s) {
+    pivmin *= s;
+    double pp = 1.0, p = (a[0] - x) * s;
     if (fabs(p) < pivmin) p = -pivmin;
     int cnt = p < 0.0 ? 1 : 0;
     auto step = [&](double ai, double bi) {
@@ -62,8 +68,8 @@ __device__ inline int sturm_count_fast(const double *a, const double *b, int n, 
         double a8[8], b8[8];  // the operands ahead of the chain
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-            a8[q] = a[i + q] - x;
-            b8[q] = b[i + q];
+            a8[q] = (a[i + q] - x) * s;
+            b8[q] = b[i + q] * s;
         }
 #pragma unroll
         for (int q = 0; q < 8; q++) step(a8[q], b8[q]);
@@ -74,8 +80,14 @@ __device__ inline int sturm_count_fast(const double *a, const double *b, int n, 
             pp *= f;
         }
     }
-    for (; i < n; i++) step(a[i] - x, b[i]);
+    for (; i < n; i++) step((a[i] - x) * s, b[i] * s);
     return cnt;
+}
+
+// The power of two s with 1 <= amax * s < 2.
+__device__ inline double tridiag_scale(double amax) {
+    const int e = min(max((__double2hiint(amax) >> 20) & 0x7ff, 1), 2045);
+    return __hiloint2double((2046 - e) << 20, 0);
 }
 
 // Bracket width, relative to |T|, above which the counts of a multisection use
@@ -101,14 +113,16 @@ __device__ inline double tridiag_eig(const double *a, const double *b, int n, in
     hi += pad;
     amax = fmax(fabs(lo), fabs(hi));
     const double pivmin = 1e-300 + 2.2e-16 * 2.2e-16 * fmax(amax * amax, 1e-300);
+    const double s = tridiag_scale(amax);
     const int nt = blockDim.x;
     if (threadIdx.x < 2) first[threadIdx.x] = nt;
     __syncthreads();
     for (int round = 0; round < 40; round++) {
         if (hi - lo <= 2.0 * 2.2e-16 * fmax(fabs(lo), fabs(hi)) + 1e-300) break;
         const double x = lo + (hi - lo) * (double)(threadIdx.x + 1) / (double)(nt + 1);
-        const int c = !EXACT || hi - lo > kFastBracket * amax ? sturm_count_fast(a, b, n, x, pivmin)
-                                                              : sturm_count(a, b, n, x, pivmin);
+        const int c = !EXACT || hi - lo > kFastBracket * amax
+                          ? sturm_count_fast(a, b, n, x, pivmin, s)
+                          : sturm_count(a, b, n, x, pivmin);
         // first point whose count exceeds j
         int *f = &first[round & 1];
         if (c > j) atomicMin(f, (int)threadIdx.x);
@@ -368,13 +382,15 @@ __device__ inline void tridiag_eigs_warp(const double *a, const double *b, int n
     hi += pad;
     const double am = fmax(fabs(lo), fabs(hi));
     const double pivmin = 1e-300 + 2.2e-16 * 2.2e-16 * fmax(am * am, 1e-300);
+    const double scale = tridiag_scale(am);
     for (int j = (int)(threadIdx.x >> 5); j < m; j += nw) {
         double l = lo, h = hi;
         for (int round = 0; round < 96; round++) {
             if (h - l <= 2.0 * 2.2e-16 * fmax(fabs(l), fabs(h)) + 1e-300) break;
             const double x = l + (h - l) * (double)(lane + 1) / 33.0;
-            const int c = !EXACT || h - l > kFastBracket * am ? sturm_count_fast(a, b, n, x, pivmin)
-                                                              : sturm_count(a, b, n, x, pivmin);
+            const int c = !EXACT || h - l > kFastBracket * am
+                              ? sturm_count_fast(a, b, n, x, pivmin, scale)
+                              : sturm_count(a, b, n, x, pivmin);
             const unsigned below = __ballot_sync(0xffffffffu, c <= j);
             const int t = below == 0xffffffffu ? 32 : __ffs(~below) - 1;
             const double nl = t == 0 ? l : l + (h - l) * (double)t / 33.0;
