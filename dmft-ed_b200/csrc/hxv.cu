@@ -654,7 +654,11 @@ __global__ void __launch_bounds__(256, kRvBlocks) k_hxv_rv(const HxvArgs<T> a) {
 constexpr uint32_t kLeanZero = 255u;
 
 // MODE 0: plain product; 1: fused Lanczos step (u and its alpha).  MB: CTAs
-// of NT threads per SM the register budget is set for.
+// of NT threads per SM the register budget is set for.  The large CTA (NT above
+// 256) takes a sector over from k_hxv_global and keeps its digits: the three
+// parts of the diagonal are added in that kernel's order and the diagonal
+// product is rounded before the first hop (the others add the column's two parts
+// once per tile and leave it to the compiler which product an fma takes).
 template <typename T, int KU, int KD, int MODE, int MB = kRvBlocks, int NT = 256>
 __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
                                                     const uint32_t *__restrict__ eux) {
@@ -662,10 +666,12 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
     constexpr int NC = 16 / sizeof(T);
     constexpr int NV = 16 / sizeof(T);
     using T2 = typename Pair<T>::type;
+    constexpr bool BIG = NT > 256;
     static_assert(KU <= 8 && KD <= 8, "hop counts above 8 use k_hxv_rv");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ T spv[256];
     __shared__ __align__(16) T cdg[NC][1 << kMaxNorb];
+    __shared__ T ndd[BIG ? NC : 1];  // bath energies of the columns
     __shared__ __align__(16) uint32_t noff[NC][8];
     __shared__ __align__(16) T nval[NC][8];
 
@@ -738,10 +744,14 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
                 const uint32_t cc = DM_IN(cg - q * dimdw, dimdw) ? cg - q * dimdw : 0u;
                 const unsigned id = a.wd[cc] & imask;
                 const T dd = a.dd[cc];
-                for (int iu = 0; iu < ni; iu++)
-                    cdg[tid][iu] = dd + a.dint[a.dswap ? id * ni + iu : iu * ni + id];
+                for (int iu = 0; iu < ni; iu++) {
+                    const T di = a.dint[a.dswap ? id * ni + iu : iu * ni + id];
+                    cdg[tid][iu] = BIG ? di : dd + di;
+                }
+                if (BIG) ndd[tid] = dd;
             } else {
                 for (int iu = 0; iu < ni; iu++) cdg[tid][iu] = T(0);
+                if (BIG) ndd[tid] = T(0);
             }
         }
         for (int t = tid; t < NC * 8; t += bd) {
@@ -807,8 +817,9 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
                 for (int j = 0; j < NC; j++) {
                     x0[j] = sw ? xb[j] : xa[j];
                     x1[j] = sw ? xa[j] : xb[j];
-                    acc[j][0] = (du2.x + cdg[j][iu0]) * x0[j];
-                    acc[j][1] = (du2.y + cdg[j][iu1]) * x1[j];
+                    const T d0 = BIG ? du2.x + ndd[j] : du2.x, d1 = BIG ? du2.y + ndd[j] : du2.y;
+                    acc[j][0] = (d0 + cdg[j][iu0]) * x0[j];
+                    acc[j][1] = (d1 + cdg[j][iu1]) * x1[j];
                 }
             }
             // 3. row hops: NC-wide gathers from the tile, fixed count
@@ -827,7 +838,8 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
                         for (int j = 0; j < NC; j++) xg[j] = T(0);
                     }
 #pragma unroll
-                    for (int j = 0; j < NC; j++) acc[j][i] += v * xg[j];
+                    for (int j = 0; j < NC; j++)
+                        acc[j][i] = BIG ? fma(v, xg[j], acc[j][i]) : acc[j][i] + v * xg[j];
                 }
             }
             // v_{k-1} rows: issued here, where the hop-table registers are free
@@ -859,8 +871,10 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
                 }
 #pragma unroll
                 for (int e = 0; e < KD; e++) {
-                    acc[j][0] += vv[e] * nb[j][e].x;
-                    acc[j][1] += vv[e] * nb[j][e].y;
+                    acc[j][0] = BIG ? fma(vv[e], nb[j][e].x, acc[j][0])
+                                    : acc[j][0] + vv[e] * nb[j][e].x;
+                    acc[j][1] = BIG ? fma(vv[e], nb[j][e].y, acc[j][1])
+                                    : acc[j][1] + vv[e] * nb[j][e].y;
                 }
             }
             // 5. Lanczos combination, store, alpha partial
@@ -1099,12 +1113,12 @@ __global__ void __launch_bounds__(256, 4) k_hxv_lean1(const HxvArgs<T> a,
 
 // ---------------------------------------------------------------------------
 // k_hxv_global: the same product for sectors whose columns do not fit in
-// shared memory (DimUp x 16 bytes above the 224 KB a tile may take, or above
-// 200 KB where k_hxv_lean does not serve the sector: Ns >= 17 near half filling).  One thread per element, in index order (a warp holds
-// consecutive rows of one column): the up hops gather from the element's own
-// column in global memory (a column is at most a few hundred KB, served from
-// L1/L2), the down hops read whole neighbour columns (coalesced), the tables
-// are the ELL ones of the other kernels.
+// shared memory (DimUp x 16 bytes above 200 KB: Ns >= 16 near half filling, but
+// for the one sector of the large CTA above).  One thread per element, in index
+// order (a warp holds consecutive rows of one column): the up hops gather from
+// the element's own column in global memory (a column is at most a few hundred
+// KB, served from L1/L2), the down hops read whole neighbour columns (coalesced),
+// the tables are the ELL ones of the other kernels.
 template <typename T, bool LZ>
 __global__ void __launch_bounds__(256) k_hxv_global(const HxvArgs<T> a) {
     if (LZ) {
@@ -1231,14 +1245,18 @@ struct HxvCfg {
     int nc, vw, threads;
     size_t smem;
     int grid;
-    bool big;     // one tile per SM: k_hxv_lean with kBigThreads threads
+    bool big;     // k_hxv_lean with one CTA of kBigThreads threads per SM
     bool global;  // the columns do not fit in shared memory: k_hxv_global
 };
 
-// One CTA of 768 threads (80 registers) per SM for tiles of more than 200 KB:
-// Ns=16 at half filling has columns of 12,870 rows, 206 KB a tile, and its FP64
-// product takes 2.48 ms against 5.01 ms with the columns in global memory (the
-// vectors, 1.3 GB each, are 0.40 ms of HBM).
+// One CTA of 768 threads (80 registers) per SM for tiles of more than 200 KB, up
+// to what fits beside the kernel's 2,912 bytes of tables (the limit is 227 KB;
+// kBigTile leaves 3 KB), where lean_shape holds.  Up to Ns=20 that is one sector,
+// the half-filled one of 16 sites of one orbital, (8,8): its columns are 12,870
+// rows, 206 KB a tile, and the words of every other class of 16 sites have nine
+// hops or more.  Its FP64 product takes 2.44 ms against 5.01 ms with the columns
+// in global memory (the vectors, 1.3 GB each, are 0.40 ms of HBM).  Forced on any
+// sector that lean_shape takes by DMFTED_HXV_KERNEL=4.
 constexpr size_t kBigTile = 224 * 1024;
 constexpr int kBigThreads = 768;
 
@@ -1269,10 +1287,10 @@ static HxvCfg hxv_config(dmfted_ctx *c, const SectorView &s, const HxvArgs<T> &a
     const int64_t ncols = a.dimdw * nstack;
     g.nc = 16 / (int)sizeof(T);  // one 16-byte gather serves the whole tile
     const size_t tile = (size_t)a.dimup * sizeof(T) * g.nc;
-    // a tile above 200 KB, up to what one CTA can take beside 4 KB of tables,
-    // runs with one large CTA per SM in k_hxv_lean; otherwise the columns
-    // stay in global memory
-    g.big = tile > (size_t)200 * 1024 && tile <= kBigTile && lean_shape<T>(c, a, g.vw);
+    // a tile above 200 KB runs with one large CTA per SM in k_hxv_lean if that
+    // kernel serves the sector; otherwise the columns stay in global memory
+    g.big = (tile > (size_t)200 * 1024 || c->tune_hxv == 4) && tile <= kBigTile &&
+            lean_shape<T>(c, a, g.vw);
     g.global = (tile > (size_t)200 * 1024 && !g.big) || c->tune_hxv == 3;
     if (g.global) {
         // one thread per element
@@ -1345,16 +1363,17 @@ static void launch_lean_mb(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, 
 // latency hiding pays more than the registers.  DMFTED_HXV_OCC=2 keeps two.
 template <typename T, int KU, int KD, int MODE>
 static void launch_lean_k(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int nvec) {
-    if (g.big) launch_lean_mb<T, KU, KD, MODE, 1, kBigThreads>(c, a, g, nvec);
-    else if (c->tune_occ == 2) launch_lean_mb<T, KU, KD, MODE, kRvBlocks>(c, a, g, nvec);
+    if (c->tune_occ == 2) launch_lean_mb<T, KU, KD, MODE, kRvBlocks>(c, a, g, nvec);
     else launch_lean_mb<T, KU, KD, MODE, 3>(c, a, g, nvec);
 }
 
-// Hop counts padded to 7 or 8 (rows and columns independently).
+// Hop counts padded to 7 or 8 (rows and columns independently); to 8 for the
+// large CTA, whose sector has fewer only where a coupling vanishes.
 template <typename T, int MODE>
 static void launch_lean(dmfted_ctx *c, const HxvArgs<T> &a, const HxvCfg &g, int nvec) {
     const bool u8 = a.ku_max > 7, d8 = a.kd_max > 7;
-    if (u8 && d8) launch_lean_k<T, 8, 8, MODE>(c, a, g, nvec);
+    if (g.big) launch_lean_mb<T, 8, 8, MODE, 1, kBigThreads>(c, a, g, nvec);
+    else if (u8 && d8) launch_lean_k<T, 8, 8, MODE>(c, a, g, nvec);
     else if (u8) launch_lean_k<T, 8, 7, MODE>(c, a, g, nvec);
     else if (d8) launch_lean_k<T, 7, 8, MODE>(c, a, g, nvec);
     else launch_lean_k<T, 7, 7, MODE>(c, a, g, nvec);
