@@ -657,6 +657,7 @@ int dmfted_init(const dmfted_params *p, const double *hloc, dmfted_ctx **out) {
         if (const char *e = getenv("DMFTED_BATCH_BUDGET_MB")) c->batch_budget = atoll(e) << 20;
         if (const char *e = getenv("DMFTED_FT_EIGS_FP32")) c->ft_eigs_fp32 = atoi(e) != 0;
         if (const char *e = getenv("DMFTED_BATCH_CHAINS_FP32")) c->batch_chains_fp32 = atoi(e) != 0;
+        if (const char *e = getenv("DMFTED_CHAINS_ONCHIP")) c->onchip_max = atoi(e);
         if (const char *e = getenv("DMFTED_BATCH_CLUSTER_MIN"))
             c->batch_cluster_min = std::max<int64_t>(1, atoll(e));
         DM_CUDA(cudaSetDevice(c->device));

@@ -111,8 +111,9 @@ inline void launch_persistent(dmfted_ctx *c, void (*kern)(KArgs...), int CL, int
 }
 
 // ---- onchip.cu -------------------------------------------------------------
-// CTAs a job needs to keep its vectors on chip (0: it does not fit 16).
-int oc_need(const dmfted_ctx *c, int nup, int ndw);
+// CTAs a job needs to keep its vectors on chip (0: it does not fit the largest
+// cluster).
+int oc_need(dmfted_ctx *c, int nup, int ndw);
 // The chains that fit on chip, in one launch; CL: CTAs of the shared ones
 // (raised to what the largest needs).
 void run_chains_onchip(dmfted_ctx *c, int CL, std::vector<ChainJob> jobs, double *alpha,

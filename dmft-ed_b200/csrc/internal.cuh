@@ -260,6 +260,8 @@ struct dmfted_ctx {
     int64_t batch_max_dim = 1 << 17;
     int64_t batch_budget = 0;             // bytes of Krylov bases per launch (0: a third of free)
     int64_t batch_cluster_min = 1024;     // states per CTA for a job shared by a cluster
+    int onchip_max = 16;                  // CTAs an on-chip chain may take (0: none, k_batch_chains)
+    int onchip_16 = -1;                   // whether a cluster of 16 of them fits the device (-1: not asked)
     // autotuner of the batched launches (batch.cu): cluster size per job-shape
     // key, measured on first use; the log keeps every measurement.  Opt-in
     // (DMFTED_AUTOTUNE=1): the job mix of a DMFT loop shifts over its first

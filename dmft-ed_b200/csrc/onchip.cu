@@ -145,16 +145,8 @@ __global__ void __launch_bounds__(kOcThreads, 1)
     }
 }
 
-int oc_need(const dmfted_ctx *c, int nup, int ndw) {
-    const OcShape o = oc_shape(c, nup, ndw);
-    for (int cl = 1; cl <= 16; cl *= 2)
-        if (oc_fits(o.R, o.D, cl, o.wr, o.wc, 1 << c->norb)) return cl;
-    return 0;
-}
-
 template <int CL>
-static void launch_chains(dmfted_ctx *c, int nbig, int nj, size_t smem, double *alpha,
-                              double *beta, int *nsteps, double *norm2, int64_t nslots) {
+static void chains_attr(dmfted_ctx *c) {
     static bool attr[64] = {false};
     if (!attr[c->device & 63]) {
         DM_CUDA(cudaFuncSetAttribute(k_chains_onchip<CL>,
@@ -162,6 +154,48 @@ static void launch_chains(dmfted_ctx *c, int nbig, int nj, size_t smem, double *
                                      (int)kOcMaxSmem));
         attr[c->device & 63] = true;
     }
+}
+
+// Whether the device takes a cluster of 16 CTAs with their full shared memory:
+// it is above the portable size, and a device with fewer SMs per GPC (or a
+// partition of one) has no room for it.
+static bool sixteen_fit(dmfted_ctx *c) {
+    if (c->onchip_16 < 0) {
+        chains_attr<16>(c);
+        DM_CUDA(cudaFuncSetAttribute(k_chains_onchip<16>,
+                                     cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 16;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(kOcThreads);
+        cfg.dynamicSmemBytes = kOcMaxSmem;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_chains_onchip<16>, &cfg) != cudaSuccess) {
+            (void)cudaGetLastError();
+            n = 0;
+        }
+        c->onchip_16 = n > 0;
+    }
+    return c->onchip_16 != 0;
+}
+
+int oc_need(dmfted_ctx *c, int nup, int ndw) {
+    const OcShape o = oc_shape(c, nup, ndw);
+    for (int cl = 1; cl <= std::min(c->onchip_max, 16); cl *= 2)
+        if (oc_fits(o.R, o.D, cl, o.wr, o.wc, 1 << c->norb))
+            return cl < 16 || sixteen_fit(c) ? cl : 0;
+    return 0;
+}
+
+template <int CL>
+static void launch_chains(dmfted_ctx *c, int nbig, int nj, size_t smem, double *alpha,
+                          double *beta, int *nsteps, double *norm2, int64_t nslots) {
+    chains_attr<CL>(c);
     launch_persistent(c, k_chains_onchip<CL>, CL, nbig + div_up(nj - nbig, CL), kOcThreads, smem,
                       batch_tables<double>(c), reinterpret_cast<const ChainJob *>(c->bjobs.p), nbig,
                       nj, reinterpret_cast<unsigned *>(c->bint.p), (const double *)c->states64.p,
@@ -172,6 +206,7 @@ static void launch_chains(dmfted_ctx *c, int nbig, int nj, size_t smem, double *
 void run_chains_onchip(dmfted_ctx *c, int CL, std::vector<ChainJob> jobs, double *alpha,
                        double *beta, int *nsteps, double *norm2, int64_t nslots) {
     auto dims = [&](const ChainJob &J) { return c->binom[J.tnup] * c->binom[J.tndw]; };
+    while (CL > 1 && (CL > c->onchip_max || (CL > 8 && !sixteen_fit(c)))) CL /= 2;
     for (const ChainJob &J : jobs) CL = std::max(CL, oc_need(c, J.tnup, J.tndw));
     auto shared = [&](const ChainJob &J) {
         return CL > 1 && (oc_need(c, J.tnup, J.tndw) > 1 || dims(J) >= c->batch_cluster_min * CL);
