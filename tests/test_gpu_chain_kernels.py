@@ -1,6 +1,8 @@
 """The two kernels of the batched Green's-function chains -- vectors on chip
-(k_chains_onchip) and in L2 (k_batch_chains) -- against each other: solves whose
-chains split between both, and the largest chains a cluster of 16 holds."""
+(k_chains_onchip) and in L2 (k_batch_chains) -- against each other and across
+the cluster sizes: chains with spin exchange and pair hopping (always through
+L2), without (either kernel), solves whose chains split between both, and the
+largest chains a cluster of 16 holds."""
 import os
 
 import numpy as np
@@ -35,6 +37,21 @@ def solve(env, norb, nbath, nspin, sectors, total=1, jhflag=0, seed=31):
 # the same eigenvectors, chains with compensated sums over other splits: the bar
 # of the cluster sizes against one CTA (test_gpu_batch.py)
 BAR = 1e-11
+
+
+@pytest.mark.parametrize("cluster", ["1", "2", "4", "8", "16"])
+@pytest.mark.parametrize("jhflag", [0, 1])
+def test_chains_through_l2_match_across_cluster_sizes(jhflag, cluster):
+    base = {"DMFTED_CHAINS_ONCHIP": "0", "DMFTED_BATCH_CLUSTER_MIN": "8",
+            "DMFTED_BATCH_CLUSTER_EIGS": "1"}
+    args = (2, 2, 2, None, 16, jhflag)
+    one, _ = solve(dict(base, DMFTED_BATCH_CLUSTER_GF="1"), *args)
+    many, _ = solve(dict(base, DMFTED_BATCH_CLUSTER_GF=cluster), *args)
+    assert np.abs(many - one).max() <= BAR
+    if not jhflag:  # the same solve on chip
+        chip, _ = solve({"DMFTED_BATCH_CLUSTER_GF": cluster, "DMFTED_BATCH_CLUSTER_MIN": "8",
+                         "DMFTED_BATCH_CLUSTER_EIGS": "1"}, *args)
+        assert np.abs(chip - one).max() <= BAR
 
 
 @pytest.mark.parametrize("nbath,sector", [
