@@ -958,6 +958,41 @@ static int tuned_cluster(dmfted_ctx *c, const char *kind, const char *override_e
     return best;
 }
 
+// The third stream beside the main one: it starts after what the main stream
+// holds when the guard is made, run() queues work on it, and join() lets the main
+// stream wait for it.  Left by an exception, the guard waits for it itself, since
+// buffers the work uses may be reused or freed next.
+struct ThirdStream {
+    dmfted_ctx *c;
+    bool joined = false;
+    explicit ThirdStream(dmfted_ctx *cc) : c(cc) {
+        if (!c->ev_fork3) DM_CUDA(cudaEventCreateWithFlags(&c->ev_fork3, cudaEventDisableTiming));
+        if (!c->ev_join3) DM_CUDA(cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming));
+        if (!c->stream3) DM_CUDA(cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking));
+        DM_CUDA(cudaEventRecord(c->ev_fork3, c->stream));
+        DM_CUDA(cudaStreamWaitEvent(c->stream3, c->ev_fork3, 0));
+    }
+    ~ThirdStream() {
+        if (!joined) cudaStreamSynchronize(c->stream3);
+    }
+    ThirdStream(const ThirdStream &) = delete;
+    ThirdStream &operator=(const ThirdStream &) = delete;
+    template <typename F>
+    void run(F f) {
+        struct Swap {
+            dmfted_ctx *c;
+            explicit Swap(dmfted_ctx *cc) : c(cc) { std::swap(c->stream, c->stream3); }
+            ~Swap() { std::swap(c->stream, c->stream3); }
+        } swap(c);
+        f();
+    }
+    void join() {
+        DM_CUDA(cudaEventRecord(c->ev_join3, c->stream3));
+        DM_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join3, 0));
+        joined = true;
+    }
+};
+
 // One launch over the jobs [j0, j1) of the queue; the job table holds the
 // whole queue, each wave has its own counter.
 template <typename T, int CL>
@@ -1098,22 +1133,10 @@ static void batch_eigs_cl(dmfted_ctx *c, const std::vector<int> &list,
         // their own queue, instead of after the clusters' (the eigensolve
         // phase of the Ns=10 finite-temperature solve: 23.3 -> 20.3 ms).
         if (CL >= 16 && nbig > 0 && j0 + nbig < j1 && c->stream2) {
-            if (!c->ev_fork3) DM_CUDA(cudaEventCreateWithFlags(&c->ev_fork3, cudaEventDisableTiming));
-            if (!c->ev_join3) DM_CUDA(cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming));
-            if (!c->stream3) DM_CUDA(cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking));
-            DM_CUDA(cudaEventRecord(c->ev_fork3, c->stream));
-            DM_CUDA(cudaStreamWaitEvent(c->stream3, c->ev_fork3, 0));
+            ThirdStream third(c);
             run(CL, j0, nbig, j0 + nbig, (int)w);
-            std::swap(c->stream, c->stream3);
-            try {
-                run(1, j0 + nbig, 0, j1, kMaxWaves + (int)w);
-            } catch (...) {
-                std::swap(c->stream, c->stream3);
-                throw;
-            }
-            std::swap(c->stream, c->stream3);
-            DM_CUDA(cudaEventRecord(c->ev_join3, c->stream3));
-            DM_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join3, 0));
+            third.run([&] { run(1, j0 + nbig, 0, j1, kMaxWaves + (int)w); });
+            third.join();
         } else {
             run(CL, j0, nbig, j1, (int)w);
         }
@@ -1154,11 +1177,11 @@ void batch_eigs(dmfted_ctx *c, const std::vector<int> &list, const std::vector<i
 }
 
 template <typename T, int CL>
-static void run_batch_chains(dmfted_ctx *c, int nbig, int nj, double *alpha, double *beta,
-                             int *nsteps, double *norm2, int64_t nslots) {
+static void run_batch_chains(dmfted_ctx *c, const ChainQueue &q, int nbig, int nj, double *alpha,
+                             double *beta, int *nsteps, double *norm2, int64_t nslots) {
     launch_persistent(c, k_batch_chains<T, CL>, CL, nbig + div_up(nj - nbig, CL), kBatchThreads, 0,
-                      batch_tables<T>(c), reinterpret_cast<const ChainJob *>(c->bjobs.p), nbig, nj,
-                      reinterpret_cast<unsigned *>(c->bint.p), (const double *)c->states64.p,
+                      batch_tables<T>(c), (const ChainJob *)q.jobs, nbig, nj, q.next,
+                      (const double *)c->states64.p,
                       reinterpret_cast<T *>(c->bwork.p), alpha, beta, nsteps, norm2,
                       c->p.lanc_gf_threshold,
                       BatchCaps{(int64_t)(c->bwork.n / sizeof(T)), 0, 0, (int64_t)c->states64.n,
@@ -1166,23 +1189,21 @@ static void run_batch_chains(dmfted_ctx *c, int nbig, int nj, double *alpha, dou
 }
 
 template <typename T>
-static void run_batch_chains_cl(dmfted_ctx *c, int CL, const std::vector<ChainJob> &jobs,
-                                double *alpha, double *beta, int *nsteps, double *norm2,
-                                int64_t nslots) {
+static void run_batch_chains_cl(dmfted_ctx *c, int CL, const ChainQueue &q,
+                                const std::vector<ChainJob> &jobs, double *alpha, double *beta,
+                                int *nsteps, double *norm2, int64_t nslots) {
     const int nj = (int)jobs.size();
-    DM_CUDA(cudaMemcpyAsync(c->bjobs.p, jobs.data(), nj * sizeof(ChainJob), cudaMemcpyHostToDevice,
-                            c->stream));
-    DM_CUDA(cudaMemsetAsync(c->bint.p, 0, 2 * sizeof(int), c->stream));
+    q.fill(c, jobs);
     int nbig = 0;  // sorted by size: the chains a cluster shares come first
     while (CL > 1 && nbig < nj &&
            c->binom[jobs[nbig].tnup] * c->binom[jobs[nbig].tndw] >= c->batch_cluster_min * CL)
         nbig++;
     switch (CL) {
-        case 16: run_batch_chains<T, 16>(c, nbig, nj, alpha, beta, nsteps, norm2, nslots); break;
-        case 8: run_batch_chains<T, 8>(c, nbig, nj, alpha, beta, nsteps, norm2, nslots); break;
-        case 4: run_batch_chains<T, 4>(c, nbig, nj, alpha, beta, nsteps, norm2, nslots); break;
-        case 2: run_batch_chains<T, 2>(c, nbig, nj, alpha, beta, nsteps, norm2, nslots); break;
-        default: run_batch_chains<T, 1>(c, 0, nj, alpha, beta, nsteps, norm2, nslots); break;
+        case 16: run_batch_chains<T, 16>(c, q, nbig, nj, alpha, beta, nsteps, norm2, nslots); break;
+        case 8: run_batch_chains<T, 8>(c, q, nbig, nj, alpha, beta, nsteps, norm2, nslots); break;
+        case 4: run_batch_chains<T, 4>(c, q, nbig, nj, alpha, beta, nsteps, norm2, nslots); break;
+        case 2: run_batch_chains<T, 2>(c, q, nbig, nj, alpha, beta, nsteps, norm2, nslots); break;
+        default: run_batch_chains<T, 1>(c, q, 0, nj, alpha, beta, nsteps, norm2, nslots); break;
     }
 }
 
@@ -1218,8 +1239,8 @@ void batch_chains_gf(dmfted_ctx *c, const std::vector<ChainRec> &recs, int preci
     c->bscal.alloc((size_t)2 * nrec * kChainStride + nrec);
     double *alpha = c->bscal.p, *beta = alpha + (size_t)nrec * kChainStride;
     double *norm2 = beta + (size_t)nrec * kChainStride;
-    c->bint.alloc(2 + nrec);
-    int *nsteps = c->bint.p + 2;
+    c->bint.alloc(4 + nrec);
+    int *nsteps = c->bint.p + 4;
     std::vector<ChainJob> jobs;
     std::vector<char> batched(nrec, 0);
     size_t work = 0;
@@ -1257,19 +1278,35 @@ void batch_chains_gf(dmfted_ctx *c, const std::vector<ChainRec> &recs, int preci
             (fp64 && !c->jterms && oc_need(c, J.tnup, J.tndw) > 0 ? onchip : rest).push_back(J);
         if (!rest.empty()) c->bwork.alloc(work * es);
         const int prec = fp64 ? DMFTED_FP64 : DMFTED_MIXED;
-        for (const std::vector<ChainJob> *part : {&onchip, &rest}) {
-            if (part->empty()) continue;
+        auto run_part = [&](const std::vector<ChainJob> &part) {
             int64_t dmax = 0;
-            for (const ChainJob &J : *part)
+            for (const ChainJob &J : part)
                 dmax = std::max<int64_t>(dmax, c->binom[J.tnup] * c->binom[J.tndw]);
-            const bool oc = part == &onchip;
+            const bool oc = &part == &onchip;
+            // each list has its own job records and queue counters
+            ChainJob *recs0 = reinterpret_cast<ChainJob *>(c->bjobs.p);
+            const ChainQueue q{oc ? recs0 : recs0 + onchip.size(),
+                               reinterpret_cast<unsigned *>(c->bint.p) + (oc ? 0 : 2)};
             tuned_cluster(c, oc ? "chains" : "chains-L2", "DMFTED_BATCH_CLUSTER_GF",
-                          chain_cluster(c, (int)part->size(), dmax), (int64_t)part->size(), dmax,
+                          chain_cluster(c, (int)jobs.size(), dmax), (int64_t)part.size(), dmax,
                           prec, [&](int cl) {
-                              if (oc) run_chains_onchip(c, cl, *part, alpha, beta, nsteps, norm2, nrec);
-                              else if (fp64) run_batch_chains_cl<double>(c, cl, *part, alpha, beta, nsteps, norm2, nrec);
-                              else run_batch_chains_cl<float>(c, cl, *part, alpha, beta, nsteps, norm2, nrec);
+                              if (oc) run_chains_onchip(c, cl, q, part, alpha, beta, nsteps, norm2, nrec);
+                              else if (fp64) run_batch_chains_cl<double>(c, cl, q, part, alpha, beta, nsteps, norm2, nrec);
+                              else run_batch_chains_cl<float>(c, cl, q, part, alpha, beta, nsteps, norm2, nrec);
                           });
+        };
+        if (!onchip.empty() && !rest.empty() && !c->autotune && c->stream2) {
+            // both at once, the L2 chains on the third stream: either list alone
+            // leaves SMs idle once its long chains are few (the two chains of the
+            // (4,2) sector of 12 sites: 7.5 ms one after the other, 5.0 ms
+            // at once, and 5.0 ms both through L2)
+            ThirdStream third(c);
+            third.run([&] { run_part(rest); });
+            run_part(onchip);
+            third.join();
+        } else {
+            if (!onchip.empty()) run_part(onchip);
+            if (!rest.empty()) run_part(rest);
         }
     }
     // chains too large for one CTA: the grid-wide recurrence, two at a time

@@ -63,6 +63,17 @@ struct BatchCaps {
     int64_t work, vec, aux, states, slots, lock;
 };
 
+// Where a list of chains keeps its job records and its two queue counters.
+struct ChainQueue {
+    ChainJob *jobs;
+    unsigned *next;
+    void fill(dmfted_ctx *c, const std::vector<ChainJob> &list) const {
+        DM_CUDA(cudaMemcpyAsync(jobs, list.data(), list.size() * sizeof(ChainJob),
+                                cudaMemcpyHostToDevice, c->stream));
+        DM_CUDA(cudaMemsetAsync(next, 0, 2 * sizeof(unsigned), c->stream));
+    }
+};
+
 struct EigsJob {
     int nup, ndw;
     int neigen, kmax;
@@ -116,7 +127,7 @@ inline void launch_persistent(dmfted_ctx *c, void (*kern)(KArgs...), int CL, int
 int oc_need(dmfted_ctx *c, int nup, int ndw);
 // The chains that fit on chip, in one launch; CL: CTAs of the shared ones
 // (raised to what the largest needs).
-void run_chains_onchip(dmfted_ctx *c, int CL, std::vector<ChainJob> jobs, double *alpha,
-                       double *beta, int *nsteps, double *norm2, int64_t nslots);
+void run_chains_onchip(dmfted_ctx *c, int CL, const ChainQueue &q, std::vector<ChainJob> jobs,
+                       double *alpha, double *beta, int *nsteps, double *norm2, int64_t nslots);
 
 }  // namespace dmfted

@@ -193,18 +193,17 @@ int oc_need(dmfted_ctx *c, int nup, int ndw) {
 }
 
 template <int CL>
-static void launch_chains(dmfted_ctx *c, int nbig, int nj, size_t smem, double *alpha,
-                          double *beta, int *nsteps, double *norm2, int64_t nslots) {
+static void launch_chains(dmfted_ctx *c, const ChainQueue &q, int nbig, int nj, size_t smem,
+                          double *alpha, double *beta, int *nsteps, double *norm2, int64_t nslots) {
     chains_attr<CL>(c);
     launch_persistent(c, k_chains_onchip<CL>, CL, nbig + div_up(nj - nbig, CL), kOcThreads, smem,
-                      batch_tables<double>(c), reinterpret_cast<const ChainJob *>(c->bjobs.p), nbig,
-                      nj, reinterpret_cast<unsigned *>(c->bint.p), (const double *)c->states64.p,
-                      alpha, beta, nsteps, norm2, c->p.lanc_gf_threshold,
+                      batch_tables<double>(c), (const ChainJob *)q.jobs, nbig, nj, q.next,
+                      (const double *)c->states64.p, alpha, beta, nsteps, norm2, c->p.lanc_gf_threshold,
                       BatchCaps{0, 0, 0, (int64_t)c->states64.n, nslots});
 }
 
-void run_chains_onchip(dmfted_ctx *c, int CL, std::vector<ChainJob> jobs, double *alpha,
-                       double *beta, int *nsteps, double *norm2, int64_t nslots) {
+void run_chains_onchip(dmfted_ctx *c, int CL, const ChainQueue &q, std::vector<ChainJob> jobs,
+                       double *alpha, double *beta, int *nsteps, double *norm2, int64_t nslots) {
     auto dims = [&](const ChainJob &J) { return c->binom[J.tnup] * c->binom[J.tndw]; };
     while (CL > 1 && (CL > c->onchip_max || (CL > 8 && !sixteen_fit(c)))) CL /= 2;
     for (const ChainJob &J : jobs) CL = std::max(CL, oc_need(c, J.tnup, J.tndw));
@@ -218,15 +217,13 @@ void run_chains_onchip(dmfted_ctx *c, int CL, std::vector<ChainJob> jobs, double
         const OcShape o = oc_shape(c, jobs[i].tnup, jobs[i].tndw);
         smem = std::max(smem, oc_smem(o.R, o.D, i < nbig ? CL : 1, o.wr, o.wc, 1 << c->norb));
     }
-    DM_CUDA(cudaMemcpyAsync(c->bjobs.p, jobs.data(), nj * sizeof(ChainJob), cudaMemcpyHostToDevice,
-                            c->stream));
-    DM_CUDA(cudaMemsetAsync(c->bint.p, 0, 2 * sizeof(int), c->stream));
+    q.fill(c, jobs);
     switch (CL) {
-        case 16: launch_chains<16>(c, nbig, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
-        case 8: launch_chains<8>(c, nbig, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
-        case 4: launch_chains<4>(c, nbig, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
-        case 2: launch_chains<2>(c, nbig, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
-        default: launch_chains<1>(c, 0, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
+        case 16: launch_chains<16>(c, q, nbig, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
+        case 8: launch_chains<8>(c, q, nbig, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
+        case 4: launch_chains<4>(c, q, nbig, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
+        case 2: launch_chains<2>(c, q, nbig, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
+        default: launch_chains<1>(c, q, 0, nj, smem, alpha, beta, nsteps, norm2, nslots); break;
     }
 }
 

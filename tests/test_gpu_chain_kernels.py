@@ -13,7 +13,7 @@ import dmfted
 pytestmark = pytest.mark.gpu
 
 
-def solve(env, norb, nbath, nspin, sectors, total=1, jhflag=0, seed=31):
+def solve(env, norb, nbath, nspin, sectors, total=1, jhflag=0, seed=31, reps=0):
     rng = np.random.default_rng(seed)
     e = rng.uniform(-1.0, 1.0, (nspin, norb, nbath))
     v = 0.5 + rng.uniform(-0.1, 0.1, (nspin, norb, nbath))
@@ -27,8 +27,16 @@ def solve(env, norb, nbath, nspin, sectors, total=1, jhflag=0, seed=31):
                                   lanc_nstates_total=total)
         with dmfted.EDSolver(p) as s:
             idx = None if sectors is None else [s.sector_index(*n) for n in sectors]
-            s.ed_solve(np.concatenate([e.reshape(-1), v.reshape(-1)]), sectors=idx)
-            return s.ed_get_gimp_matsubara(), s.launch_count()
+            bath = np.concatenate([e.reshape(-1), v.reshape(-1)])
+            s.ed_solve(bath, sectors=idx)
+            g, n = s.ed_get_gimp_matsubara(), s.launch_count()
+            if not reps:
+                return g, n
+            times = []
+            for _ in range(reps):
+                s.ed_solve(bath, sectors=idx)
+                times.append(s.timings()["gf_ms"])
+            return min(times)
     finally:
         for k, val in old.items():
             os.environ.pop(k) if val is None else os.environ.__setitem__(k, val)
@@ -69,3 +77,10 @@ def test_chains_split_between_the_kernels(nbath, sector):
     assert np.abs(eight - l2).max() <= BAR
     if sector[1] == 2:  # one launch each for the two kernels
         assert n_mixed == n_l2 + 1
+
+
+def test_split_chains_run_at_once():
+    # one list after the other takes 1.5 times as long as both chains through L2
+    split, l2 = (solve(env, 1, 11, 1, [(4, 2)], reps=9)
+                 for env in ({}, {"DMFTED_CHAINS_ONCHIP": "0"}))
+    assert split <= 1.25 * l2
