@@ -42,18 +42,19 @@ __device__ inline int sturm_count(const double *a, const double *b, int n, doubl
 // Sturm count: number of eigenvalues of the n x n tridiagonal (a, b[1..n-1])
 // below x, as sign changes of the leading principal minors
 //   p_i = (a_i - x) p_{i-1} - b_i^2 p_{i-2},
-// a zero pivot ratio |p_i / p_{i-1}| < pivmin counting as a negative one.  T, x
-// and pivmin are multiplied by s, a power of two that brings |T| near one
-// (tridiag_scale), and the minors rescaled by a power of two every eight steps:
-// eight pivots, even all at pivmin, then stay within the range of FP64 at every
-// energy unit (unscaled, eight steps of |T| = 1e-38 underflow to a wrong count),
-// and both scalings are exact.  Two FP64 operations, a compare and a select per
-// step (45 cycles) against the 320 of the division in sturm_count; the two agree
-// unless x is within rounding of an eigenvalue.
-__device__ inline int sturm_count_fast(const double *a, const double *b, int n, double x,
-                                       double pivmin, double s) {
-    pivmin *= s;
-    double pp = 1.0, p = (a[0] - x) * s;
+// a zero pivot ratio |p_i / p_{i-1}| < pivmin counting as a negative one.  The
+// minors are rescaled by a power of two every eight steps, and T, x and pivmin are
+// multiplied by s, a power of two too (tridiag_scale): eight pivots, even all at
+// pivmin, then stay within the range of FP64 at every energy unit (unscaled,
+// eight steps of |T| = 1e-38 underflow to a wrong count).  SCALED = false: s = 1.
+// Two FP64 operations, a compare and a select per step (45 cycles) against the
+// 320 of the division in sturm_count; the two agree unless x is within rounding
+// of an eigenvalue.
+template <bool SCALED>
+__device__ inline int sturm_count_minors(const double *a, const double *b, int n, double x,
+                                         double pivmin, double s) {
+    if (SCALED) pivmin *= s;
+    double pp = 1.0, p = SCALED ? (a[0] - x) * s : a[0] - x;
     if (fabs(p) < pivmin) p = -pivmin;
     int cnt = p < 0.0 ? 1 : 0;
     auto step = [&](double ai, double bi) {
@@ -68,8 +69,8 @@ __device__ inline int sturm_count_fast(const double *a, const double *b, int n, 
         double a8[8], b8[8];  // the operands ahead of the chain
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-            a8[q] = (a[i + q] - x) * s;
-            b8[q] = b[i + q] * s;
+            a8[q] = SCALED ? (a[i + q] - x) * s : a[i + q] - x;
+            b8[q] = SCALED ? b[i + q] * s : b[i + q];
         }
 #pragma unroll
         for (int q = 0; q < 8; q++) step(a8[q], b8[q]);
@@ -80,12 +81,22 @@ __device__ inline int sturm_count_fast(const double *a, const double *b, int n, 
             pp *= f;
         }
     }
-    for (; i < n; i++) step((a[i] - x) * s, b[i] * s);
+    for (; i < n; i++) {
+        if (SCALED) step((a[i] - x) * s, b[i] * s);
+        else step(a[i] - x, b[i]);
+    }
     return cnt;
 }
+__device__ inline int sturm_count_fast(const double *a, const double *b, int n, double x,
+                                       double pivmin, double s) {
+    return s == 1.0 ? sturm_count_minors<false>(a, b, n, x, pivmin, s)
+                    : sturm_count_minors<true>(a, b, n, x, pivmin, s);
+}
 
-// The power of two s with 1 <= amax * s < 2.
+// The power of two s with 1 <= amax * s < 2; 1 where nine pivots at pivmin =
+// 4.8e-32 amax^2 (3e-33 each at 0.25) or of 4 amax stay within the range unscaled.
 __device__ inline double tridiag_scale(double amax) {
+    if (amax >= 0.25 && amax <= 1e18) return 1.0;
     const int e = min(max((__double2hiint(amax) >> 20) & 0x7ff, 1), 2045);
     return __hiloint2double((2046 - e) << 20, 0);
 }
