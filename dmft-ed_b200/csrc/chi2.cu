@@ -11,17 +11,19 @@
 // at compile time (up to kChi2Levels) a thread's 1/(e_k^2 + w^2) and its sums of
 // chi^2 and of both derivatives stay in registers; V_k^2 and 2 V_k, the same for
 // every point, multiply the sums once at the end.  The reciprocal is a Newton
-// iteration from the single-precision one, to the last bit of the division that
-// it replaces, without a branch between the NB chains.  The sums are folded
-// compensated, one warp per sum, in a fixed order.  What bounds it: the FP64
-// pipe's latency at four or five CTAs per SM.  4096 sets of 9 levels, 1000
-// points: 72 us against 133 us with the sums in shared memory and divisions; the
-// 20 FP64 operations per level and point are 42 us of the pipe.  Largest errors
-// against 64-bit references over 24 inputs, of the norm: chi^2 2.9e-16 (3.5e-16
-// before), gradient 3.49e-16 (3.53e-16); means 2.07e-16 (2.04e-16) and 2.30e-16
-// (2.22e-16).  Every accumulation is one rounded product sum and one addition: a
-// gradient term folded in by two chained fma is 2 us faster, with errors of 3.53e-16
-// and 2.33e-16.
+// iteration from the single-precision one, without a branch between the NB chains.
+// The sums are folded compensated, one warp per sum, in a fixed order.  What bounds
+// it: the FP64 pipe's latency at the few CTAs per SM that the registers allow.
+// 4096 sets of 9 levels, 1000 points: 72 us against 133 us with the sums in shared
+// memory and divisions (k_chi2); the 20 FP64 operations per level and point are
+// 42 us of the pipe.
+// Errors against extended precision over 81,920 sets (1 to 16 levels, 200 to 1500
+// points), relative to the value or the gradient's norm, this kernel and k_chi2:
+// chi^2 4.145e-16 and 4.167e-16 in the mean, gradient 5.111e-16 and 5.124e-16.
+// They come from the residual g - Delta, so Im Delta is summed with one rounding
+// per level (fma of V^2 and the reciprocal; a rounded product and an addition:
+// 4.183e-16 and 5.140e-16), and every term of a final sum is formed first and added
+// with one rounding.
 #include <algorithm>
 
 #include "internal.cuh"
@@ -29,16 +31,24 @@
 
 namespace dmfted {
 
-// Registers hold 3 NB + 1 FP64 values: the CTAs per SM that leave no or few
-// spills (9 levels: 69 us with four, 77 us with five).
+// Registers hold 3 NB + 1 FP64 values; more CTAs per SM hide latency until the
+// spills cost more.  4096 sets, 1000 points, us a call with 2 / 3 / 4 / 5 CTAs:
+// 5 levels 49 / 49 / 49 / 47, 8 levels 74 / 74 / 71 / 76, 10 levels 102 / 90 / 88 /
+// 115, 11 levels 110 / 99 / 100 / 144, 13 levels 125 / 113 / 127 / 208, 15 levels
+// 143 / 141 / 186 / 258, 16 levels 150 / 155 / 222 / 296; up to four levels the
+// choice makes no difference.  At 11 levels four are taken for small batches (512
+// sets are one wave of four per SM: 12.3 against 14.4 us).
 constexpr int kChi2Levels = 16;
 constexpr int kChi2Threads = 128;
+constexpr int chi2_ctas(int nb) { return nb <= 5 ? 5 : nb <= 11 ? 4 : nb <= 15 ? 3 : 2; }
 
 // 1/d: Newton iteration from the approximate single-precision reciprocal, whose
 // argument and result change format by integer shifts of the bit pattern (the
 // conversion instructions share the FP64 pipe's slow path).  Each of the two
 // steps doubles the 22 bits of the start; the last one leaves its own rounding.
-// For d within about 1e-29 .. 1e29, where the shifts hold (chi2_in_range).
+// Against the division: the same bits for all of 1e9 random d, and within one ulp
+// (0.8 % of the cases) where d is within 4096 ulp of a power of two.  For d within
+// about 1e-29 .. 1e29, where the shifts hold (chi2_in_range).
 __device__ __forceinline__ bool chi2_in_range(double d) {
     const int hi = __double2hiint(d);
     return hi > 0x3a000000 && hi < 0x46000000;
@@ -53,7 +63,7 @@ __device__ __forceinline__ double chi2_recip(double d) {
 }
 
 template <int NB>
-__global__ void __launch_bounds__(kChi2Threads, NB <= 4 ? 6 : NB <= 8 ? 5 : NB <= 12 ? 4 : 3)
+__global__ void __launch_bounds__(kChi2Threads, chi2_ctas(NB))
     k_chi2_reg(int L, const double *__restrict__ a, const double *__restrict__ x,
                const double *__restrict__ g, const double *__restrict__ w, double *chi2,
                double *grad) {
@@ -91,11 +101,11 @@ __global__ void __launch_bounds__(kChi2Threads, NB <= 4 ? 6 : NB <= 8 ? 5 : NB <
         for (int k = 0; k < NB; k++) {
             const double t = pv2[k] * inv[k];
             dre = fma(pe[k], t, dre);
-            dim += t;
+            dim = fma(pv2[k], inv[k], dim);
         }
         const double Rr = gn.x + dre, Ri = fma(om, dim, gn.y);
         const double Wr = Rr * iw, Wi = Ri * iw;
-        s0 = fma(Rr, Wr, fma(Ri, Wi, s0));
+        s0 += fma(Rr, Wr, Ri * Wi);
 #pragma unroll
         for (int k = 0; k < NB; k++) {
             // dDelta/de = v^2 r^2 ; dDelta/dV = 2 v r, with r = 1/(i om - e)
