@@ -191,17 +191,18 @@ __global__ void k_interleave_split(const double *z, double *re, double *im, int6
 // The same with the complex side in pinned host memory, whole complex numbers
 // per access.
 __global__ void __launch_bounds__(256) k_stage_in(const double2 *z, double *re, double *im, int64_t n) {
-    pdl_begin();
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const double2 v = z[i];
         re[i] = v.x;
         im[i] = v.y;
     }
+    pdl_trigger();
 }
 __global__ void __launch_bounds__(256) k_stage_out(const double *re, const double *im, double2 *z,
                                                    int64_t n) {
-    pdl_begin();
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
         z[i] = make_double2(re[i], im[i]);
@@ -646,6 +647,7 @@ int dmfted_init(const dmfted_params *p, const double *hloc, dmfted_ctx **out) {
         c->device = p->device;
         if (const char *e = getenv("DMFTED_HXV_NC")) c->tune_nc = atoi(e);
         if (const char *e = getenv("DMFTED_HXV_KERNEL")) c->tune_hxv = atoi(e);
+        if (const char *e = getenv("DMFTED_LAUNCH_OVERLAP")) c->overlap = atoi(e) != 0;
         if (const char *e = getenv("DMFTED_HXV_OCC")) c->tune_occ = atoi(e);
         if (const char *e = getenv("DMFTED_ELL_GROUP")) c->tune_ell_group = std::max(1, std::min(32, atoi(e)));
         if (const char *e = getenv("DMFTED_MIXED_TOL32")) c->mixed_tol32 = atof(e);

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256, kHxvMinBlocks) k_hxv(const HxvArgs<T> a) 
     __shared__ T sval[NC][kMaxW];
     __shared__ int64_t soff[NC][kMaxW];
 
-    pdl_begin();
+    pdl_wait();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
     }
@@ -311,6 +311,7 @@ __global__ void __launch_bounds__(256, kHxvMinBlocks) k_hxv(const HxvArgs<T> a) 
         }
     }
     if (LZ) {
+        pdl_trigger();
         CSum arr[1] = {dot};
         double tot[1];
         if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__(256, kRvBlocks) k_hxv_rv(const HxvArgs<T> a) {
     __shared__ __align__(16) T nval[NC][kMaxW];
     __shared__ int scnt[NC];
 
-    pdl_begin();
+    pdl_wait();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
     }
@@ -628,6 +629,7 @@ __global__ void __launch_bounds__(256, kRvBlocks) k_hxv_rv(const HxvArgs<T> a) {
         }
     }
     if (LZ) {
+        pdl_trigger();
         CSum arr[1] = {dot};
         double tot[1];
         if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {
@@ -675,7 +677,7 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
     __shared__ __align__(16) uint32_t noff[NC][8];
     __shared__ __align__(16) T nval[NC][8];
 
-    pdl_begin();
+    pdl_wait();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
     }
@@ -906,6 +908,7 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
         }
     }
     if (MODE == 1) {
+        pdl_trigger();
         CSum arr[1] = {dot};
         double tot[1];
         if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {
@@ -937,7 +940,7 @@ __global__ void __launch_bounds__(256, 4) k_hxv_lean1(const HxvArgs<T> a,
     __shared__ T ndd[NC];
     __shared__ int ncnt[NC];
 
-    pdl_begin();
+    pdl_wait();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
     }
@@ -1103,6 +1106,7 @@ __global__ void __launch_bounds__(256, 4) k_hxv_lean1(const HxvArgs<T> a,
         }
     }
     if (MODE == 1) {
+        pdl_trigger();
         CSum arr[1] = {dot};
         double tot[1];
         if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {

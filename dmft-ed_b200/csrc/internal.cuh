@@ -247,6 +247,7 @@ struct dmfted_ctx {
     // H*v kernel: 0 automatic, 1 k_hxv, 2 k_hxv_rv, 3 k_hxv_global, 4 the large
     // CTA of k_hxv_lean (in place of that kernel's other forms)
     int tune_hxv = 0;
+    bool overlap = true;                  // launches that overlap the previous kernel's end
     int tune_occ = 3;                     // k_hxv_lean CTAs per SM (3: 80 registers; 2: 128)
     int tune_ell_group = 0;               // lanes per hop-table balance group (0: 8)
     dmfted::DBuf<double> d_wm, d_wr;      // Matsubara / real-axis grids
@@ -532,15 +533,21 @@ inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 int num_sms(dmfted_ctx *c);
 
 // ---- launches that overlap the end of the stream's previous kernel ----------
-// A kernel launched by launch_overlapped starts when every CTA of the previous
-// kernel in the stream has begun (its launch latency and its scheduling run under
-// that kernel's last wave) and calls pdl_begin() before it touches memory, which
-// returns once the previous kernel has completed and its writes are visible.  A
-// previous kernel that does not trigger, or another operation in between, makes
-// it an ordinary launch.
-__device__ __forceinline__ void pdl_begin() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// A kernel launched by launch_overlapped is scheduled when every CTA of the
+// previous kernel in the stream has called pdl_trigger() or ended, so that its
+// launch latency runs under that kernel's end, and calls pdl_wait() before it
+// touches memory, which returns once the previous kernel has completed and its
+// writes are visible.  The previous kernel triggers when its CTA's elements are
+// done, before the grid reduction: a CTA scheduled earlier takes its SM among the
+// previous kernel's, and a grid of one or two CTAs per SM then lands unevenly (a
+// Lanczos step of the (5,3) sector of 11 sites: 19.2 us triggered at the start,
+// 13.0 at the end of the elements, 16.4 without overlap).  Plain products end
+// there and do not trigger.  After another operation it is an ordinary launch.
+__device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_trigger() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <typename... KArgs, typename... Args>
@@ -553,7 +560,7 @@ inline void launch_overlapped(dmfted_ctx *c, void (*kern)(KArgs...), dim3 grid, 
     cfg.stream = c->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].val.programmaticStreamSerializationAllowed = c->overlap ? 1 : 0;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     DM_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));

@@ -54,7 +54,7 @@ template <typename T, int VW>
 __global__ void __launch_bounds__(kRedThreads) k_lz_update(T *u, const T *scur, int64_t n,
                                                            LanczosScalars lz, int k, double thr,
                                                            double *partials, unsigned *counter) {
-    pdl_begin();
+    pdl_wait();
     if (lz.status[ST_DONE]) return;
     const double coef = lz.alpha[k] * lz.scale[k];
     CSum s;
@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(kRedThreads) k_lz_update(T *u, const T *scur, 
             *reinterpret_cast<uint4 *>(u + i) = qu;
         }
     }
+    pdl_trigger();
     CSum arr[1] = {s};
     double tot[1];
     if (grid_reduce<1>(arr, partials, counter, tot)) {
