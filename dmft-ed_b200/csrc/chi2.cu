@@ -19,7 +19,7 @@
 // 42 us of the pipe.
 // Errors against extended precision over 81,920 sets (1 to 16 levels, 200 to 1500
 // points), relative to the value or the gradient's norm, this kernel and k_chi2:
-// chi^2 4.145e-16 and 4.167e-16 in the mean, gradient 5.111e-16 and 5.124e-16.
+// chi^2 4.145e-16 and 4.167e-16 in the mean, gradient 5.110e-16 and 5.124e-16.
 // They come from the residual g - Delta, so Im Delta is summed with one rounding
 // per level (fma of V^2 and the reciprocal; a rounded product and an addition:
 // 4.183e-16 and 5.140e-16), and every term of a final sum is formed first and added
@@ -99,8 +99,7 @@ __global__ void __launch_bounds__(kChi2Threads, chi2_ctas(NB))
         // 1/(i om - e) = (-e - i om) inv; the signs and -om go outside the sums
 #pragma unroll
         for (int k = 0; k < NB; k++) {
-            const double t = pv2[k] * inv[k];
-            dre = fma(pe[k], t, dre);
+            dre = fma(pv2[k], pe[k] * inv[k], dre);
             dim = fma(pv2[k], inv[k], dim);
         }
         const double Rr = gn.x + dre, Ri = fma(om, dim, gn.y);
