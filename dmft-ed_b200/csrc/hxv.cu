@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(256, kHxvMinBlocks) k_hxv(const HxvArgs<T> a) 
     __shared__ T sval[NC][kMaxW];
     __shared__ int64_t soff[NC][kMaxW];
 
+    if (LZ) pdl_trigger();
     pdl_wait();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
@@ -311,7 +312,6 @@ __global__ void __launch_bounds__(256, kHxvMinBlocks) k_hxv(const HxvArgs<T> a) 
         }
     }
     if (LZ) {
-        pdl_trigger();
         CSum arr[1] = {dot};
         double tot[1];
         if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {
@@ -367,6 +367,7 @@ __global__ void __launch_bounds__(256, kRvBlocks) k_hxv_rv(const HxvArgs<T> a) {
     __shared__ __align__(16) T nval[NC][kMaxW];
     __shared__ int scnt[NC];
 
+    if (LZ) pdl_trigger();
     pdl_wait();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
@@ -629,7 +630,6 @@ __global__ void __launch_bounds__(256, kRvBlocks) k_hxv_rv(const HxvArgs<T> a) {
         }
     }
     if (LZ) {
-        pdl_trigger();
         CSum arr[1] = {dot};
         double tot[1];
         if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {
@@ -677,6 +677,7 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
     __shared__ __align__(16) uint32_t noff[NC][8];
     __shared__ __align__(16) T nval[NC][8];
 
+    if (LZ) pdl_trigger();
     pdl_wait();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
@@ -908,7 +909,6 @@ __global__ void __launch_bounds__(NT, MB) k_hxv_lean(const HxvArgs<T> a,
         }
     }
     if (MODE == 1) {
-        pdl_trigger();
         CSum arr[1] = {dot};
         double tot[1];
         if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {
@@ -940,6 +940,7 @@ __global__ void __launch_bounds__(256, 4) k_hxv_lean1(const HxvArgs<T> a,
     __shared__ T ndd[NC];
     __shared__ int ncnt[NC];
 
+    if (LZ) pdl_trigger();
     pdl_wait();
     if (LZ) {
         if (a.status[0]) return;  // chain finished: every later step is a no-op
@@ -1106,7 +1107,6 @@ __global__ void __launch_bounds__(256, 4) k_hxv_lean1(const HxvArgs<T> a,
         }
     }
     if (MODE == 1) {
-        pdl_trigger();
         CSum arr[1] = {dot};
         double tot[1];
         if (grid_reduce<1>(arr, a.partials, a.counter, tot)) {

@@ -537,12 +537,17 @@ int num_sms(dmfted_ctx *c);
 // previous kernel in the stream has called pdl_trigger() or ended, so that its
 // launch latency runs under that kernel's end, and calls pdl_wait() before it
 // touches memory, which returns once the previous kernel has completed and its
-// writes are visible.  The previous kernel triggers when its CTA's elements are
-// done, before the grid reduction: a CTA scheduled earlier takes its SM among the
-// previous kernel's, and a grid of one or two CTAs per SM then lands unevenly (a
-// Lanczos step of the (5,3) sector of 11 sites: 19.2 us triggered at the start,
-// 13.0 at the end of the elements, 16.4 without overlap).  Plain products end
-// there and do not trigger.  After another operation it is an ordinary launch.
+// writes are visible.  After another operation it is an ordinary launch.
+// Where a kernel triggers decides which SMs its successor finds free.  A product
+// released at the start of the update before it takes its SMs among the update's
+// CTAs, and a grid of one or two CTAs per SM then lands unevenly: the update
+// triggers when its CTA's elements are done, before the grid reduction (a Lanczos
+// step of the (5,3) sector of 11 sites: 19.2 us with the release at the start, 14.6
+// at the end of the elements, 16.4 without overlap).  The product releases the
+// update, whose many CTAs fit in anywhere, at its own start: released at the end
+// of its elements a step alone is shorter (13.0 us), but two chains side by side
+// then fall into step on some sectors (chains of (6,6) at 12 sites in FP64 7.8
+// against 7.0 ms).  Plain products do not trigger.
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
