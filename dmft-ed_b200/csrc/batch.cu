@@ -530,7 +530,8 @@ __device__ void eigs_job(const BatchTables<T> &tb, BatchSmem<T> &sm, double *dyn
     // steps: while the decay of the worst estimate (over its target) since the
     // last test predicts more than four intervals to go, every other one is
     // left out, so the test that sees convergence is the one the fixed schedule
-    // would run.
+    // would run, unless convergence more than doubles its pace right after a test
+    // (the solve then ends ncheck steps later, with a smaller residual).
     int next = ncheck, at_prev = 0;
     double worst_prev = 0.0;
     for (int k = 0; k < J.kmax; k++) {
@@ -853,9 +854,9 @@ void gf_add_chain(dmfted_ctx *c, int nlanc, const double *alanc, const double *b
 // batch_cluster_min states per CTA, to amortise the cluster barriers; 16, the
 // non-portable cluster size, from 32 per CTA), or DMFTED_BATCH_CLUSTER_EIGS.
 // Only sectors that give every CTA that many states are shared; smaller ones
-// run one per CTA.  (Eight CTAs are faster on the Ns=10 workload, 18.1 against
-// 23.4 ms of eigensolves, but end in other last digits: quantities that vanish
-// by symmetry are then other rounding noise.)
+// run one per CTA.  With the small sectors beside the clusters of 16 (below), 16
+// and 8 CTAs are even on the Ns=10 workload: diagonalisation of four baths 19.1 /
+// 17.7 / 18.4 / 22.2 ms with 16, 19.9 / 16.5 / 17.7 / 24.6 with 8.
 static int eigs_cluster(const dmfted_ctx *c, int64_t dmax) {
     const int64_t per = c->batch_cluster_min;
     if (const char *e = getenv("DMFTED_BATCH_CLUSTER_EIGS")) {
@@ -870,7 +871,7 @@ static int eigs_cluster(const dmfted_ctx *c, int64_t dmax) {
 // chains of the Ns=10 workload took 35.0 ms with pairs against 38.9 ms one per
 // CTA), more only while the chains leave SMs idle; or DMFTED_BATCH_CLUSTER_GF.
 // On-chip chains take at least the CTAs their largest needs (four at 52,920
-// states: 8.8 ms; eight 11.3 ms).
+// states; eight for all took 14 to 43 ms where four took 10 to 23 ms).
 static int chain_cluster(dmfted_ctx *c, int njobs, int64_t dmax) {
     const int64_t per = c->batch_cluster_min;
     if (const char *e = getenv("DMFTED_BATCH_CLUSTER_GF")) {
@@ -1131,7 +1132,7 @@ static void batch_eigs_cl(dmfted_ctx *c, const std::vector<int> &list,
         // Clusters of 16 leave SMs idle (at most seven or eight fit the GPCs): the
         // sectors of one CTA each start there at once, on the third stream with
         // their own queue, instead of after the clusters' (the eigensolve
-        // phase of the Ns=10 finite-temperature solve: 23.3 -> 20.3 ms).
+        // phase of one Ns=10 finite-temperature solve: 23.3 -> 20.3 ms).
         if (CL >= 16 && nbig > 0 && j0 + nbig < j1 && c->stream2) {
             ThirdStream third(c);
             run(CL, j0, nbig, j0 + nbig, (int)w);

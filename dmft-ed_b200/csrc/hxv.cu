@@ -1311,8 +1311,10 @@ static HxvCfg hxv_config(dmfted_ctx *c, const SectorView &s, const HxvArgs<T> &a
 }
 
 // Lanczos steps, and plain products of at most a CTA per SM, overlap the end of
-// the stream's previous kernel (a step of Ns=12 24 -> 21 us); larger plain
-// products back to back lose 1 % by it (CTAs that wait hold the SMs' slots).
+// the stream's previous kernel: a step of (6,6) at 12 sites 24 -> 21 us, a plain
+// product of (5,3) at 10 sites 6.2 -> 4.2 us.  Larger plain products gain 1 to 3 %
+// back to back, but lose 1 % when other work lies between them (two orbitals, (6,6)
+// at 12 sites 13.73 -> 13.85 us), which is how they are called.
 template <bool LZ, typename... KArgs, typename... Args>
 static void launch_product(dmfted_ctx *c, void (*kern)(KArgs...), const HxvCfg &g, int nvec,
                            Args &&...args) {

@@ -10,9 +10,11 @@ namespace dmfted {
 // ---- a chain (chain_job in batch.cu) with its vectors on chip ---------------
 // One Lanczos step: u = sc H x - b_k scp v_prev over v_prev's registers and
 // alpha (first barrier), then x -> v_prev, w = u - alpha sc x -> x and |w|
-// (second barrier).  The chains of the two-orbital Ns=10 workload (72 of up to
-// 52,920 states, four CTAs each) take 9.7 ms against 15.1 ms with the vectors
-// in L2; the two of the Ns=8 scan (4,900 and 3,920 states) 1.1 against 2.1 ms.
+// (second barrier).  Green's-function phase of the two-orbital Ns=10 solve at
+// finite temperature (88 to 200 chains of up to 52,920 states, four CTAs for the
+// large ones), four baths: 17.3 / 10.0 / 12.9 / 23.0 ms against 24.8 / 18.5 / 18.6 /
+// 33.9 with the vectors in L2; of the Ns=8 scan (4,900 and 3,920 states) 1.26
+// against 2.1 ms; a chain of 108,900 states on sixteen CTAs 8.4 against 12.2 ms.
 template <int CL>
 __device__ void chain_job_oc(const BatchTables<double> &tb, OcSums<CL> &sums, unsigned char *dyn,
                              const ChainJob &J, const double *states64, double *alpha,

@@ -4,9 +4,11 @@
 // one CTA).  The vector is the DimUp x DimDw matrix; each CTA keeps a contiguous
 // block of columns in shared memory, with the row hop table of the sector and
 // the column hop tables of its own columns: a Lanczos step reads nothing from
-// L2.  Every element's arithmetic is that of the jobs in batch.cu, and the sums
-// do not depend on the split of the elements (CSum::add_product), so both give
-// the same numbers to the last digit: a bath fit's path hangs on it.
+// L2.  Rows are the up words, columns the down words; up to kOcThreads rows.
+// Every element's arithmetic is that of the jobs in batch.cu and the sums hardly
+// depend on the split of the elements (CSum::add_product): G(i w_n) of 32 solves
+// (4 to 14 sites, one to three orbitals, one to sixteen CTAs) was equal in every
+// bit, or to 6e-16, between the two.
 //  * Row hops gather from the element's own column in this CTA's shared memory.
 //    A thread owns one row and walks over columns, four at a time, so that one
 //    table entry and one coupling serve four gathers.
@@ -17,8 +19,7 @@
 //    of columns shares its high sites and most hops stay inside it (a warp's
 //    256-byte read of another CTA's shared memory takes 13.6 cycles of the SM
 //    against 2 for its own; copies of the vector in L2, read there instead,
-//    were slower for their latency: 11.5 against 8.6 ms for the chains of the
-//    Ns=10 workload).
+//    took a third longer for their latency).
 //  * The previous vector lives in registers: kOcSlots elements per thread.
 //  * A sum over the job is one barrier: every warp writes its partial into all
 //    CTAs of the cluster, and after the barrier every warp folds the partials
@@ -42,9 +43,7 @@ constexpr int kOcThreads = 512;               // 128 registers per thread
 constexpr int kOcWarps = kOcThreads / 32;
 constexpr int kOcCols = 4;                    // columns per thread and pass
 constexpr int kOcSlots = 32;                  // elements per thread in registers
-constexpr int kOcBlocks = kOcSlots / kOcCols;
 constexpr size_t kOcMaxSmem = 216 * 1024;     // dynamic shared memory of a job
-
 
 // Shared memory of a job of R rows (at most wr hops each) and D columns (wc)
 // on CL CTAs, each array padded to 16 bytes, and whether a job fits: its

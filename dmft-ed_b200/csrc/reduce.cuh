@@ -26,9 +26,10 @@ struct CSum {
         hi = s;
         lo += e;
     }
-    // add(x * y) with the product exact (its rounding error goes to lo): a sum of
-    // products then does not depend on how its terms are split over threads, to
-    // its last digit, nor on where the compiler fuses the product.
+    // add(x * y) with the product's rounding error in lo, whatever the compiler
+    // fuses.  lo itself is summed in FP64, so the sum of products can still differ
+    // between two splits of its terms, but only where hi + lo lies within some 1e-16
+    // of its own last digit of a rounding boundary.
     __device__ __forceinline__ void add_product(double x, double y) {
         const double s = fma(x, y, hi), bb = __dadd_rn(s, -hi);
         lo = __dadd_rn(lo, __dadd_rn(__dadd_rn(hi, -__dadd_rn(s, -bb)), fma(x, y, -bb)));

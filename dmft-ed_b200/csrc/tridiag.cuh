@@ -22,10 +22,7 @@ __device__ __forceinline__ double random_start_value(int64_t i, uint64_t seed) {
 }
 
 // Sturm count: number of eigenvalues of the n x n tridiagonal (a, b[1..n-1])
-// below x.  (The division-free product form of the leading minors was
-// measured too: faster per count in a 256-thread block, but slower in the
-// batched eigensolver's 1024-thread blocks, where the counts are bound by
-// FP64 issue rather than by the latency of the division chain.)
+// below x, by the pivots of T - x.
 __device__ inline int sturm_count(const double *a, const double *b, int n, double x, double pivmin) {
     int cnt = 0;
     double q = a[0] - x;

@@ -1,6 +1,7 @@
 """The global-memory H*v (k_hxv_global) that serves sectors whose columns do
 not fit in shared memory (DimUp x 16 bytes above 200 KB: Ns >= 16 near half
-filling), against the oracle.
+filling, but for the half-filled sector of 16 sites of one orbital, which
+test_gpu_hxv_large_cta.py covers), against the oracle.
 
 Checks:
   - forced on small sectors (DMFTED_HXV_KERNEL=3), the product equals the

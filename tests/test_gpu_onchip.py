@@ -1,8 +1,8 @@
 """Batched jobs whose vectors stay on chip (one CTA or a cluster) against the
 grid-wide path on the same problems, at the shapes where the work split has its
 edges: a row count that does not divide the block, more up than down words and
-the reverse (the smaller class becomes the rows), a single column, sectors that
-need 2 to 16 CTAs."""
+the reverse (up words are always the rows), a single row, chains that need one to
+four CTAs (test_gpu_chain_kernels.py holds those that need sixteen)."""
 import os
 
 import numpy as np
